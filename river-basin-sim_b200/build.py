@@ -64,7 +64,7 @@ def needs_build() -> bool:
     if not os.path.exists(OUT):
         return True
     t = os.path.getmtime(OUT)
-    deps = (sources() + glob.glob(os.path.join(CSRC, "*.h*")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    deps = (sources() + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
             + [os.path.abspath(__file__)])  # fmt: skip
     return any(os.path.getmtime(d) > t for d in deps)
 
