@@ -658,6 +658,9 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
   __syncthreads();  // the shared tile is reused by the caller's next tile
 }
 
+#include "warp_stream.cuh"
+#include "li_stream.cuh"
+
 // The single-domain step kernel. MINB is __launch_bounds__' resident-block hint (it
 // caps registers at 65536 / (MINB * NT)).
 template <int TX, int TY, int NT, bool CH, int MINB, int SED>
@@ -715,7 +718,7 @@ cudaError_t li_step_launch_variant(const LiParams& p, int variant, cudaStream_t 
     case 2: return launch_li<64, 16, 512, false, 3>(p, s);
     case 3: return launch_li<32, 8, 256, false, 1>(p, s);
     case 4: return launch_li<32, 16, 256, false, 5>(p, s);  // at most 48 registers
-    default: return launch_li<32, 32, 512, false, 3>(p, s);
+    default: return li_stream_takes(p) ? launch_li_stream(p, s) : launch_li<32, 32, 512, false, 3>(p, s);
   }
 }
 

