@@ -265,6 +265,40 @@ __device__ __forceinline__ void any_face_flux(const Rec& L, const Rec& R, int ki
   any_face_flux(sides(L, R), kind, low, e, stage, fh, fl, fr, ft, h_l_out, h_r_out);
 }
 
+// Manning friction on the new momenta of a wet cell (hllc.py:912-939): the numerator
+// g dt n^2 |q| is zero, and the denominator exactly 1 so hu and hv stand as they are,
+// whenever n = 0 with a finite |q|^2 or the water is still with a finite g dt n^2;
+// neither the square root nor the power is needed then.
+__device__ __forceinline__ void hllc_friction(float hh, bool wet, float gdt, float n, float& hu, float& hv) {
+  const float m2 = hu * hu + hv * hv;
+  const float k = gdt * n * n;
+  if (wet && !((k == 0.0f && m2 <= FLT_MAX) || (m2 == 0.0f && k <= FLT_MAX))) {
+    const float f = k * sqrtf(m2);
+    if (!(f == 0.0f)) {
+      const float denom = 1.0f + f / pow73(hh);
+#if defined(RB_FAST_MATH)
+      const float rd = 1.0f / denom;
+      hu = hu * rd;
+      hv = hv * rd;
+#else
+      hu = div_pos(hu, denom);
+      hv = div_pos(hv, denom);
+#endif
+    }
+  }
+}
+
+// max(|u|, |v|) + sqrt(g h) of a cell (hllc.py:948-966 _reduce_wavespeed).
+__device__ __forceinline__ float wave_speed(float hh, float hu, float hv) {
+  const float cw = sqrtf(kG * rmax(hh, 0.0f));
+  const bool wet = hh > kHDry;
+#if defined(RB_FAST_MATH)
+  return wet ? rmax(fabsf(hu), fabsf(hv)) * (1.0f / (wet ? hh : 1.0f)) + cw : cw;
+#else
+  return wet ? rmax(div_if(wet, fabsf(hu), hh), div_if(wet, fabsf(hv), hh)) + cw : cw;
+#endif
+}
+
 template <int TX, int TY>
 struct HllcSmem {
   static constexpr int H = 3;                     // halo
@@ -891,26 +925,7 @@ __device__ __forceinline__ bool hllc_tile(const HllcParams& p, int bx, int by, s
       if (hh > kHDry) {
         hu = 0.5f * (g_hun[i] + g_hus[i] + dt * dhu);
         hv = 0.5f * (g_hvn[i] + g_hvs[i] + dt * dhv);
-        // friction (hllc.py:912-939): the numerator g dt n^2 |q| is zero, and the
-        // denominator exactly 1 so hu and hv stand as they are, whenever n = 0 with a
-        // finite |q|^2 or the water is still with a finite g dt n^2; neither the
-        // square root nor the power is needed then
-        const float m2 = hu * hu + hv * hv;
-        const float k = g * dt * g_n[i] * g_n[i];
-        if (!((k == 0.0f && m2 <= FLT_MAX) || (m2 == 0.0f && k <= FLT_MAX))) {
-          const float f = k * sqrtf(m2);
-          if (!(f == 0.0f)) {
-            const float denom = 1.0f + f / pow73(hh);
-#if defined(RB_FAST_MATH)
-            const float rd = 1.0f / denom;
-            hu = hu * rd;
-            hv = hv * rd;
-#else
-            hu = div_pos(hu, denom);
-            hv = div_pos(hv, denom);
-#endif
-          }
-        }
+        hllc_friction(hh, true, g * dt, g_n[i], hu, hv);
       }
       if (SRC != 0 && rain_mode == 1) {
         float comp = p.h_comp[id];
@@ -940,13 +955,7 @@ __device__ __forceinline__ bool hllc_tile(const HllcParams& p, int bx, int by, s
       p.hub[cur ^ 1][id] = hu;
       p.hvb[cur ^ 1][id] = hv;
       // hllc.py:948-966 _reduce_wavespeed on the new state
-      const float cw = sqrtf(g * rmax(hh, 0.0f));
-      const bool wet = hh > kHDry;
-#if defined(RB_FAST_MATH)
-      const float s = wet ? rmax(fabsf(hu), fabsf(hv)) * (1.0f / (wet ? hh : 1.0f)) + cw : cw;
-#else
-      const float s = wet ? rmax(div_if(wet, fabsf(hu), hh), div_if(wet, fabsf(hv), hh)) + cw : cw;
-#endif
+      const float s = wave_speed(hh, hu, hv);
       smax = s > smax ? s : smax;
       bad |= !(fabsf(hh) <= FLT_MAX) || !(fabsf(hu) <= FLT_MAX) || !(fabsf(hv) <= FLT_MAX);
     }
@@ -966,6 +975,9 @@ __device__ __forceinline__ bool hllc_tile(const HllcParams& p, int bx, int by, s
   __syncthreads();  // the shared tile is reused by the caller's next tile
   return true;
 }
+
+#include "warp_stream.cuh"
+#include "hllc_stream.cuh"
 
 // The single-domain stage kernel. Shared memory is dynamic (a 32 x 32 tile needs
 // more than the 48 KB a static array may take); __launch_bounds__ asks for two
@@ -1280,7 +1292,8 @@ cudaError_t hllc_stage_launch_exact(const HllcParams& p, int stage, int variant,
     case 4: return launch_hllc<32, 32, 512, 1, 1>(p, stage, s);
     case 7: return launch_hllc_tma<32, 32, 640>(p, stage, s);
     case 8: return launch_hllc_tma<32, 32, 512, true>(p, stage, s);
-    default: return launch_hllc<32, 32, 640, 1, 1>(p, stage, s);
+    default:
+      return hllc_stream_takes(p) ? launch_hllc_stream(p, stage, s) : launch_hllc<32, 32, 640, 1, 1>(p, stage, s);
   }
 }
 
@@ -1290,8 +1303,12 @@ cudaError_t hllc_stage_launch_exact(const HllcParams& p, int stage, int variant,
 int hllc_tiles(int ny, int nx) { return hllc_tiles_of(g_hllc_variant.load(), ny, nx); }
 
 int hllc_tiles_of(int variant, int ny, int nx) {
-  const HllcKernelVariant& v = kHllcVariants[variant >= 0 && variant < kNumHllcVariants ? variant : kDefaultHllcVariant];
-  return ((nx + v.tx - 1) / v.tx) * ((ny + v.ty - 1) / v.ty);
+  const bool known = variant >= 0 && variant < kNumHllcVariants;
+  const HllcKernelVariant& v = kHllcVariants[known ? variant : kDefaultHllcVariant];
+  const int tiles = ((nx + v.tx - 1) / v.tx) * ((ny + v.ty - 1) / v.ty);
+  // the default variant's streaming kernel, in either arithmetic, has a slot per block
+  const bool stream = (!known || variant == kDefaultHllcVariant) && hllc_stream_fits(ny, nx);
+  return stream ? std::max(tiles, hllc_stream_blocks(ny, nx)) : tiles;
 }
 
 // Ensemble: one Heun stage over the (domain, local tile) work-list of every HLLC

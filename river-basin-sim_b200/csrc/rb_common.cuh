@@ -67,6 +67,12 @@ __device__ __forceinline__ float rcp_near(float y) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
   return r;
 }
+// The approximate square root, flushing subnormals.
+__device__ __forceinline__ float sqrt_near(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 // h^(7/3) for a normal h >= H_DRY: __powf's bits without its handling of subnormals. The
 // maximum changes nothing there (the power is above 2^-24); it keeps the assembler from
 // folding a reciprocal of the result into an exponential of the negated argument, which
@@ -142,11 +148,20 @@ __device__ __forceinline__ float div_rn_by(float a, float b, float y) {
   const float q = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
   return __uint_as_float((__float_as_uint(q) & 0x7fffffffu) | (__float_as_uint(a) & 0x80000000u));
 }
-__device__ __forceinline__ float div_rn(float a, float b) {
+__device__ __forceinline__ float rcp_rn(float b) {  // the correctly rounded 1 / b, b in [2^-24, 2^64]
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-  y = __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
-  return div_rn_by(a, b, y);
+  return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
+}
+__device__ __forceinline__ float div_rn(float a, float b) { return div_rn_by(a, b, rcp_rn(b)); }
+
+// The IEEE square root for a in [2^-100, 2^100]: Markstein's residual correction of
+// a * rsqrt(a) (same paper), compared with __fsqrt_rn on all 1 677 721 601 of them.
+__device__ __forceinline__ float sqrt_rn(float a) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+  const float q = a * y;
+  return __fmaf_rn(__fmaf_rn(-q, q, a), 0.5f * y, q);
 }
 
 // rb_pow73f for x in [2^-12, 2^20], the same bits without a branch. The operations of
@@ -176,6 +191,10 @@ __device__ __forceinline__ float pow73_mid(float x) {
 }
 
 __device__ __forceinline__ float div_g(float x) { return rb_div_g(x); }  // x / g, bit for bit
+// rb_div_g for x >= 2^-99, without its other branch
+__device__ __forceinline__ float rb_div_g_mid(float x) {
+  return __fmaf_rn(x, 0x1.a1887ap-4f, x * 0x1.dcb5p-38f);
+}
 __device__ __forceinline__ bool quotient_nonneg(float n, float d) { return rb_quotient_nonneg(n, d) != 0; }
 __device__ __forceinline__ float pow73(float x) { return rb_pow73f(x); }
 __device__ __forceinline__ float pow13(float x) { return rb_pow13f(x); }

@@ -94,6 +94,31 @@ struct HllcParams {
   unsigned int *err;
 };
 
+// The row-streaming HLLC stage kernel's split (hllc_stream.cuh), the same in both
+// arithmetics: columns a warp's strip stores, rows a warp walks, blocks (one ledger slot
+// each) of a domain, and whether a domain's strips fit the ledger (a slot per 32 x 8
+// cells: all but narrow and flat domains do), the grid and 32-bit row offsets.
+constexpr int kHllcStreamCols = 26;
+// Two waves of the 16 warps an SM holds, within 11 .. 48 rows: three rows above and below
+// a chunk are overhead, and with one long wave the domain's edge strips, which check
+// bounds, end last (2048^2 dam break, fast, us per step: 196 / 190 / 191 / 228 for 19 / 28 /
+// 35 / 48 rows).
+inline int hllc_stream_rows(int ny, int nx) {
+  const long long strips = (nx + kHllcStreamCols - 1) / kHllcStreamCols;
+  const long long rows = (ny * strips + 2 * 148 * 16 - 1) / (2 * 148 * 16);
+  return (int)(rows < 11 ? 11 : (rows > 48 ? 48 : rows));
+}
+inline int hllc_stream_blocks(int ny, int nx) {
+  const int rows = hllc_stream_rows(ny, nx);
+  return ((nx + kHllcStreamCols - 1) / kHllcStreamCols) * ((ny + rows - 1) / rows);
+}
+inline bool hllc_stream_fits(int ny, int nx) {
+  const int rows = hllc_stream_rows(ny, nx);
+  const long long blocks = (long long)((nx + kHllcStreamCols - 1) / kHllcStreamCols) * ((ny + rows - 1) / rows);
+  return blocks <= (long long)((nx + 31) / 32) * ((ny + 7) / 8) && (ny + rows - 1) / rows <= 65535 &&
+         (long long)(rows + 16) * nx < (1LL << 31);
+}
+
 // The tensor maps (CUtensorMap, 128 bytes each, held opaque here) of the fields the
 // TMA-staged HLLC stage kernel copies into shared memory: both buffers of h, hu, hv
 // (the clock picks one at run time), the bed and the stage-1 state.
