@@ -36,6 +36,8 @@
 namespace rb {
 RB_ARITH_BEGIN
 
+#include "warp_stream.cuh"
+
 // hllc.py:158-165 _minmod
 #if defined(RB_FAST_MATH)
 // Fast arithmetic: minmod is the median of a, b and 0 (four min / max operations, no
@@ -55,8 +57,9 @@ __device__ __forceinline__ float dryfactor(float h0, float hm, float hp) {
   return (h0 <= kHDry || hm <= kHDry || hp <= kHDry) ? 0.0f : 1.0f;
 }
 
+#if !defined(RB_FAST_MATH)
 // hllc.py:191-256 _hllc: (mass, normal momentum, transverse momentum) flux.
-__device__ __forceinline__ void hllc_flux(float hl, float ul, float vtl, float hr, float ur, float vtr, float& f0,
+__device__ __forceinline__ void hllc_flux_any(float hl, float ul, float vtl, float hr, float ur, float vtr, float& f0,
                                           float& f1, float& f2) {
   const float g = kG;
   const float cl = sqrtf(g * rmax(hl, 0.0f));
@@ -77,12 +80,8 @@ __device__ __forceinline__ void hllc_flux(float hl, float ul, float vtl, float h
     sr = ul + 2.0f * cl;
   } else {
     const float hs = 0.5f * (cl + cr) + 0.25f * (ul - ur);
-#if defined(RB_FAST_MATH)
-    const float c_star = fabsf(hs);  // sqrt(g * max(hs * hs / g, 0)) = |hs|
-#else
     const float h_star = rmax(div_g(hs * hs), 0.0f);  // hs * hs / g
     const float c_star = sqrtf(g * h_star);
-#endif
     const float u_star = 0.5f * (ul + ur) + cl - cr;
     sl = rmin(ul - cl, u_star - c_star);
     sr = rmax(ur + cr, u_star + c_star);
@@ -92,17 +91,6 @@ __device__ __forceinline__ void hllc_flux(float hl, float ul, float vtl, float h
   const float fh_r = hr * ur;
   const float fmn_r = hr * ur * ur + 0.5f * g * hr * hr;
   float fh, fmn;
-#if defined(RB_FAST_MATH)
-  {
-    // Fast arithmetic: the three cases in one formula. With the wave speeds clamped
-    // to sl <= 0 <= sr, the HLL flux is the left flux when sl >= 0 and the right one
-    // when sr <= 0 (to rounding); sl < sr whenever one side is wet.
-    const float a = fminf(sl, 0.0f), b = fmaxf(sr, 0.0f);
-    const float inv = 1.0f / fmaxf(b - a, 1.0e-30f);
-    fh = (b * fh_l - a * fh_r + a * b * (hr - hl)) * inv;
-    fmn = (b * fmn_l - a * fmn_r + a * b * (hr * ur - hl * ul)) * inv;
-  }
-#else
   if (sl >= 0.0f) {
     fh = fh_l;
     fmn = fmn_l;
@@ -114,19 +102,12 @@ __device__ __forceinline__ void hllc_flux(float hl, float ul, float vtl, float h
     fh = (sr * fh_l - sl * fh_r + sl * sr * (hr - hl)) * inv;
     fmn = (sr * fmn_l - sl * fmn_r + sl * sr * (hr * ur - hl * ul)) * inv;
   }
-#endif
   // The contact speed s_star is read only through s_star >= 0 (hllc.py:231-238), so
   // its sign is decided without the division (quotient_nonneg).
   const float den_s = hr * (ur - sr) - hl * (ul - sl);
-#if defined(RB_FAST_MATH)
-  // fast arithmetic: the sign of the quotient from the sign of the product
-  const bool star_nonneg =
-      fabsf(den_s) > 1.0e-12f ? (sl * hr * (ur - sr) - sr * hl * (ul - sl)) * den_s >= 0.0f : ul + ur >= 0.0f;
-#else
   const bool star_nonneg = fabsf(den_s) > 1.0e-12f
                                ? quotient_nonneg(sl * hr * (ur - sr) - sr * hl * (ul - sl), den_s)
                                : 0.5f * (ul + ur) >= 0.0f;
-#endif
   const float vt = star_nonneg ? vtl : vtr;
   f0 = fh;
   f1 = fmn;
@@ -137,16 +118,7 @@ __device__ __forceinline__ void hllc_flux(float hl, float ul, float vtl, float h
 // one. Still water (hu = hv = 0) is common, and its quotients are the zero momenta
 // themselves, so such cells branch around both divisions (a zero dividend would take
 // the division's slow path); a cell with one zero momentum divides 1 in its place.
-#if defined(RB_FAST_MATH)
-// Fast arithmetic: one approximate reciprocal per wet cell.
-__device__ __forceinline__ void primitives(float h, float hu, float hv, float& u, float& v) {
-  const bool wet = h > kHDry;
-  const float r = 1.0f / (wet ? h : 1.0f);
-  u = wet ? hu * r : 0.0f;
-  v = wet ? hv * r : 0.0f;
-}
-#else
-__device__ __forceinline__ void primitives(float h, float hu, float hv, float& u, float& v) {
+__device__ __forceinline__ void primitives_any(float h, float hu, float hv, float& u, float& v) {
   const bool wet = h > kHDry;
   u = wet ? hu : 0.0f;
   v = wet ? hv : 0.0f;
@@ -156,6 +128,182 @@ __device__ __forceinline__ void primitives(float h, float hu, float hv, float& u
     if (hu != 0.0f) u = qu;
     if (hv != 0.0f) v = qv;
   }
+}
+
+// Manning friction on the new momenta of a wet cell (hllc.py:912-939): the numerator
+// g dt n^2 |q| is zero, and the denominator exactly 1 so hu and hv stand as they are,
+// whenever n = 0 with a finite |q|^2 or the water is still with a finite g dt n^2;
+// neither the square root nor the power is needed then.
+__device__ __forceinline__ void friction_any(float hh, bool wet, float gdt, float n, float& hu, float& hv) {
+  const float m2 = hu * hu + hv * hv;
+  const float k = gdt * n * n;
+  if (wet && !((k == 0.0f && m2 <= FLT_MAX) || (m2 == 0.0f && k <= FLT_MAX))) {
+    const float f = k * sqrtf(m2);
+    if (!(f == 0.0f)) {
+      const float denom = 1.0f + f / pow73(hh);
+      hu = div_pos(hu, denom);
+      hv = div_pos(hv, denom);
+    }
+  }
+}
+
+// max(|u|, |v|) + sqrt(g h) of a cell (hllc.py:948-966 _reduce_wavespeed).
+__device__ __forceinline__ float wave_speed_any(float hh, float hu, float hv) {
+  const float cw = sqrtf(kG * rmax(hh, 0.0f));
+  const bool wet = hh > kHDry;
+  return wet ? rmax(div_if(wet, fabsf(hu), hh), div_if(wet, fabsf(hv), hh)) + cw : cw;
+}
+
+#endif  // !RB_FAST_MATH
+
+// The cell and face arithmetic as the kernels evaluate it. Exact build: the values of the
+// `_any` functions above without branches, by correctly rounded divisions and square roots
+// inside a safe range (rcp_rn, div_rn, sqrt_rn); `odd` is set where an operand leaves it,
+// and the caller redoes those with the `_any` function. VOTE: every lane of the warp calls
+// (the row-streaming kernels), so a warp can skip what none of its lanes needs.
+#if defined(RB_FAST_MATH)
+// Fast arithmetic: the approximate units in their flush-to-zero forms, the star celerity as
+// |hs| (sqrt(g max(hs^2 / g, 0))), the three HLL cases in one formula (with the wave speeds
+// clamped to sl <= 0 <= sr the HLL flux is the left one when sl >= 0 and the right one when
+// sr <= 0, to rounding; sl < sr whenever one side is wet), the contact speed's sign from a
+// product, one reciprocal per cell.
+__device__ __forceinline__ void primitives_near(float h, float hu, float hv, float& u, float& v, bool&) {
+  const bool wet = h > kHDry;
+  const float r = rcp_near(wet ? h : 1.0f);
+  u = wet ? hu * r : 0.0f;
+  v = wet ? hv * r : 0.0f;
+}
+
+__device__ __forceinline__ void hllc_near(float hl, float ul, float vtl, float hr, float ur, float vtr, float& f0,
+                                          float& f1, float& f2, bool&) {
+  const float g = kG;
+  const float cl = sqrt_near(g * fmaxf(hl, 0.0f)), cr = sqrt_near(g * fmaxf(hr, 0.0f));
+  const bool dry_l = hl <= kHDry, dry_r = hr <= kHDry;
+  const float c_star = fabsf(0.5f * (cl + cr) + 0.25f * (ul - ur));
+  const float u_star = 0.5f * (ul + ur) + cl - cr;
+  float sl = fminf(ul - cl, u_star - c_star), sr = fmaxf(ur + cr, u_star + c_star);
+  if (dry_r) sl = ul - cl, sr = ul + 2.0f * cl;
+  if (dry_l) sl = ur - 2.0f * cr, sr = ur + cr;
+  const float fh_l = hl * ul, fmn_l = hl * ul * ul + 0.5f * g * hl * hl;
+  const float fh_r = hr * ur, fmn_r = hr * ur * ur + 0.5f * g * hr * hr;
+  const float a = fminf(sl, 0.0f), b = fmaxf(sr, 0.0f);
+  const float inv = rcp_near(fmaxf(b - a, 1.0e-30f));
+  const float fh = (b * fh_l - a * fh_r + a * b * (hr - hl)) * inv;
+  const float fmn = (b * fmn_l - a * fmn_r + a * b * (hr * ur - hl * ul)) * inv;
+  const float den_s = hr * (ur - sr) - hl * (ul - sl);
+  const bool star_nonneg =
+      fabsf(den_s) > 1.0e-12f ? (sl * hr * (ur - sr) - sr * hl * (ul - sl)) * den_s >= 0.0f : ul + ur >= 0.0f;
+  const bool none = dry_l && dry_r;
+  f0 = none ? 0.0f : fh;
+  f1 = none ? 0.0f : fmn;
+  f2 = none ? 0.0f : fh * (star_nonneg ? vtl : vtr);
+}
+
+template <bool VOTE>
+__device__ __forceinline__ void hllc_friction(float hh, bool wet, float gdt, float n, float& hu, float& hv) {
+  const float f = gdt * n * n * sqrt_near(hu * hu + hv * hv);
+  const float rd = rcp_near(1.0f + f * rcp_near(pow73_near(hh)));
+  if (wet) hu *= rd, hv *= rd;
+}
+
+template <bool VOTE>
+__device__ __forceinline__ float wave_speed(float hh, float hu, float hv) {
+  const float cw = sqrt_near(kG * fmaxf(hh, 0.0f));
+  const bool wet = hh > kHDry;
+  return wet ? rmax(fabsf(hu), fabsf(hv)) * rcp_near(wet ? hh : 1.0f) + cw : cw;
+}
+
+__device__ __forceinline__ void primitives(float h, float hu, float hv, float& u, float& v) {
+  bool odd;
+  primitives_near(h, hu, hv, u, v, odd);
+}
+__device__ __forceinline__ void hllc_flux(float hl, float ul, float vtl, float hr, float ur, float vtr, float& f0,
+                                          float& f1, float& f2) {
+  bool odd;
+  hllc_near(hl, ul, vtl, hr, ur, vtr, f0, f1, f2, odd);
+}
+#else
+__device__ __forceinline__ void primitives_near(float h, float hu, float hv, float& u, float& v, bool& odd) {
+  const bool wet = h > kHDry;
+  const float hs = wet ? h : 1.0f, y = rcp_rn(hs);
+  const float qu = div_rn_by(hu, hs, y), qv = div_rn_by(hv, hs, y);
+  u = wet ? qu : 0.0f;
+  v = wet ? qv : 0.0f;
+  const float m = fmaxf(fabsf(hu), fabsf(hv));
+  odd |= wet & !(div_rn_small_ok(hu) & div_rn_small_ok(hv) & (h <= 0x1p24f) & (m <= 0x1p60f));
+}
+
+__device__ __forceinline__ void hllc_near(float hl, float ul, float vtl, float hr, float ur, float vtr, float& f0,
+                                          float& f1, float& f2, bool& odd) {
+  const float g = kG;
+  const bool dry_l = hl <= kHDry, dry_r = hr <= kHDry, none = dry_l & dry_r;
+  // a dry side's celerity is not used
+  const float cl = sqrt_rn(g * (dry_l ? 1.0f : hl)), cr = sqrt_rn(g * (dry_r ? 1.0f : hr));
+  const float hs = 0.5f * (cl + cr) + 0.25f * (ul - ur);
+  const float hs2 = hs * hs;
+  const float c_star = sqrt_rn(g * rb_div_g_mid(hs2));
+  const float u_star = 0.5f * (ul + ur) + cl - cr;
+  float sl = rmin(ul - cl, u_star - c_star), sr = rmax(ur + cr, u_star + c_star);
+  if (dry_r) sl = ul - cl, sr = ul + 2.0f * cl;
+  if (dry_l) sl = ur - 2.0f * cr, sr = ur + cr;
+  const float fh_l = hl * ul, fmn_l = hl * ul * ul + 0.5f * g * hl * hl;
+  const float fh_r = hr * ur, fmn_r = hr * ur * ur + 0.5f * g * hr * hr;
+  const float gap = sr - sl, inv = rcp_rn(gap);
+  const float fh_m = (sr * fh_l - sl * fh_r + sl * sr * (hr - hl)) * inv;
+  const float fmn_m = (sr * fmn_l - sl * fmn_r + sl * sr * (hr * ur - hl * ul)) * inv;
+  const float fh = sl >= 0.0f ? fh_l : (sr <= 0.0f ? fh_r : fh_m);
+  const float fmn = sl >= 0.0f ? fmn_l : (sr <= 0.0f ? fmn_r : fmn_m);
+  // the sign of the contact speed num_s / den_s (quotient_nonneg without its rare cases)
+  const float den_s = hr * (ur - sr) - hl * (ul - sl);
+  const float num_s = sl * hr * (ur - sr) - sr * hl * (ul - sl);
+  const bool have_s = fabsf(den_s) > 1.0e-12f;
+  const bool nonneg = have_s ? (num_s == 0.0f) | ((num_s > 0.0f) == (den_s > 0.0f)) : 0.5f * (ul + ur) >= 0.0f;
+  const bool sign_ok = !have_s | (num_s == 0.0f) | (fabsf(num_s) > fabsf(den_s) * 0x1p-100f);
+  f0 = none ? 0.0f : fh;
+  f1 = none ? 0.0f : fmn;
+  f2 = none ? 0.0f : fh * (nonneg ? vtl : vtr);
+  odd |= !none & !((gap >= 0x1p-20f) & (gap <= 0x1p50f) & (dry_l | dry_r | (hs2 >= 0x1p-99f)) & sign_ok);
+}
+
+template <bool VOTE>
+__device__ __forceinline__ void hllc_friction(float hh, bool wet, float gdt, float n, float& hu, float& hv) {
+  const float m2 = hu * hu + hv * hv, k = gdt * n * n;
+  const bool need = wet & !(((k == 0.0f) & (m2 <= FLT_MAX)) | ((m2 == 0.0f) & (k <= FLT_MAX)));
+  if (!any_lane<VOTE>(need)) return;
+  const float f = k * sqrt_rn(need ? m2 : 1.0f);
+  const float den = 1.0f + div_rn(f, pow73_mid(need ? hh : 1.0f));
+  const float y = rcp_rn(den);
+  const float qu = div_rn_by(hu, den, y), qv = div_rn_by(hv, den, y);
+  const bool ok = (m2 >= 0x1p-100f) & (m2 <= 0x1p100f) & (hh <= 0x1p19f) & (f <= 0x1p40f) & (den <= 0x1p20f) &
+                  div_rn_small_ok(hu) & div_rn_small_ok(hv);
+  if (any_lane<VOTE>(need & !ok))
+    friction_any(hh, wet, gdt, n, hu, hv);
+  else if (need)
+    hu = qu, hv = qv;
+}
+
+// max(|u|, |v|) + sqrt(g h) of a cell (hllc.py:948-966 _reduce_wavespeed). The larger
+// quotient is the larger dividend's: rounding is monotonic.
+template <bool VOTE>
+__device__ __forceinline__ float wave_speed(float hh, float hu, float hv) {
+  const bool wet = hh > kHDry;
+  const float a = rmax(fabsf(hu), fabsf(hv)), hs = wet ? hh : 1.0f;
+  const bool ok = !wet | ((hh <= 0x1p24f) & (a <= 0x1p60f) & div_rn_small_ok(a));
+  if (any_lane<VOTE>(!ok | ((hh > 0.0f) & !(hh >= 0x1p-100f)))) return wave_speed_any(hh, hu, hv);
+  const float cw = hh > 0.0f ? sqrt_rn(kG * hh) : 0.0f;
+  return wet ? div_rn(a, hs) + cw : cw;
+}
+
+__device__ __forceinline__ void primitives(float h, float hu, float hv, float& u, float& v) {
+  bool odd = false;
+  primitives_near(h, hu, hv, u, v, odd);
+  if (odd) primitives_any(h, hu, hv, u, v);
+}
+__device__ __forceinline__ void hllc_flux(float hl, float ul, float vtl, float hr, float ur, float vtr, float& f0,
+                                          float& f1, float& f2) {
+  bool odd = false;
+  hllc_near(hl, ul, vtl, hr, ur, vtr, f0, f1, f2, odd);
+  if (odd) hllc_flux_any(hl, ul, vtl, hr, ur, vtr, f0, f1, f2);
 }
 #endif
 
@@ -227,11 +375,11 @@ __device__ __forceinline__ void any_face_flux(const FaceSides& F, int kind, bool
                                               float& fh, float& fl, float& fr, float& ft, float& h_l_out,
                                               float& h_r_out) {
   const float g = kG;
-  const float h_l = rmax(F.eL - F.zL, 0.0f);
-  const float h_r = rmax(F.eR - F.zR, 0.0f);
+  const float h_l = fmaxf(F.eL - F.zL, 0.0f);
+  const float h_r = fmaxf(F.eR - F.zR, 0.0f);
   const float z_star = rmax(F.zL, F.zR);
-  const float hl_star = rmax(F.eL - z_star, 0.0f);
-  const float hr_star = rmax(F.eR - z_star, 0.0f);
+  const float hl_star = fmaxf(F.eL - z_star, 0.0f);
+  const float hr_star = fmaxf(F.eR - z_star, 0.0f);
   h_l_out = h_l;
   h_r_out = h_r;
   float hl = hl_star, ul = F.nL, vl = F.tL, hr = hr_star, ur = F.nR, vr = F.tR;
@@ -263,40 +411,6 @@ __device__ __forceinline__ void any_face_flux(const Rec& L, const Rec& R, int ki
                                               float stage, float& fh, float& fl, float& fr, float& ft,
                                               float& h_l_out, float& h_r_out) {
   any_face_flux(sides(L, R), kind, low, e, stage, fh, fl, fr, ft, h_l_out, h_r_out);
-}
-
-// Manning friction on the new momenta of a wet cell (hllc.py:912-939): the numerator
-// g dt n^2 |q| is zero, and the denominator exactly 1 so hu and hv stand as they are,
-// whenever n = 0 with a finite |q|^2 or the water is still with a finite g dt n^2;
-// neither the square root nor the power is needed then.
-__device__ __forceinline__ void hllc_friction(float hh, bool wet, float gdt, float n, float& hu, float& hv) {
-  const float m2 = hu * hu + hv * hv;
-  const float k = gdt * n * n;
-  if (wet && !((k == 0.0f && m2 <= FLT_MAX) || (m2 == 0.0f && k <= FLT_MAX))) {
-    const float f = k * sqrtf(m2);
-    if (!(f == 0.0f)) {
-      const float denom = 1.0f + f / pow73(hh);
-#if defined(RB_FAST_MATH)
-      const float rd = 1.0f / denom;
-      hu = hu * rd;
-      hv = hv * rd;
-#else
-      hu = div_pos(hu, denom);
-      hv = div_pos(hv, denom);
-#endif
-    }
-  }
-}
-
-// max(|u|, |v|) + sqrt(g h) of a cell (hllc.py:948-966 _reduce_wavespeed).
-__device__ __forceinline__ float wave_speed(float hh, float hu, float hv) {
-  const float cw = sqrtf(kG * rmax(hh, 0.0f));
-  const bool wet = hh > kHDry;
-#if defined(RB_FAST_MATH)
-  return wet ? rmax(fabsf(hu), fabsf(hv)) * (1.0f / (wet ? hh : 1.0f)) + cw : cw;
-#else
-  return wet ? rmax(div_if(wet, fabsf(hu), hh), div_if(wet, fabsf(hv), hh)) + cw : cw;
-#endif
 }
 
 template <int TX, int TY>
@@ -804,19 +918,11 @@ __device__ __forceinline__ bool hllc_tile(const HllcParams& p, int bx, int by, s
     const int gi = y0 - 1 + a, gj = x0 - 1 + b;
     float beta = 1.0f;
     if (IN || (gi >= 0 && gi < ny && gj >= 0 && gj < nx)) {
-      float q_out = 0.0f;
-      const float fl = s_fxh[a][b];
-      if (fl < 0.0f) q_out = q_out - fl;
-      const float fr = s_fxh[a][b + 1];
-      if (fr > 0.0f) q_out = q_out + fr;
-      const float ft = s_fyh[a][b];
-      if (ft < 0.0f) q_out = q_out - ft;
-      const float fb = s_fyh[a + 1][b];
-      if (fb > 0.0f) q_out = q_out + fb;
-      const float out_depth = dtdx * q_out;
-      const bool out = out_depth > 0.0f;
-      const float ratio = div_if(out, s_c[a + 2][b + 2].x, out_depth);
-      if (out) beta = rclamp(ratio, 0.0f, 1.0f);
+      const float q_out = fmaxf(-s_fxh[a][b], 0.0f) + fmaxf(s_fxh[a][b + 1], 0.0f) + fmaxf(-s_fyh[a][b], 0.0f) +
+                          fmaxf(s_fyh[a + 1][b], 0.0f);
+      const float out_depth = dtdx * q_out, hc = s_c[a + 2][b + 2].x;
+      // h >= out_depth gives 1
+      if (out_depth > 0.0f && !(hc >= out_depth)) beta = rclamp(div_in_branch(hc, out_depth), 0.0f, 1.0f);
     }
     s_beta[a][b] = beta;
   }
@@ -925,7 +1031,7 @@ __device__ __forceinline__ bool hllc_tile(const HllcParams& p, int bx, int by, s
       if (hh > kHDry) {
         hu = 0.5f * (g_hun[i] + g_hus[i] + dt * dhu);
         hv = 0.5f * (g_hvn[i] + g_hvs[i] + dt * dhv);
-        hllc_friction(hh, true, g * dt, g_n[i], hu, hv);
+        hllc_friction<false>(hh, true, g * dt, g_n[i], hu, hv);
       }
       if (SRC != 0 && rain_mode == 1) {
         float comp = p.h_comp[id];
@@ -955,7 +1061,7 @@ __device__ __forceinline__ bool hllc_tile(const HllcParams& p, int bx, int by, s
       p.hub[cur ^ 1][id] = hu;
       p.hvb[cur ^ 1][id] = hv;
       // hllc.py:948-966 _reduce_wavespeed on the new state
-      const float s = wave_speed(hh, hu, hv);
+      const float s = wave_speed<false>(hh, hu, hv);
       smax = s > smax ? s : smax;
       bad |= !(fabsf(hh) <= FLT_MAX) || !(fabsf(hu) <= FLT_MAX) || !(fabsf(hv) <= FLT_MAX);
     }
@@ -976,7 +1082,6 @@ __device__ __forceinline__ bool hllc_tile(const HllcParams& p, int bx, int by, s
   return true;
 }
 
-#include "warp_stream.cuh"
 #include "hllc_stream.cuh"
 
 // The single-domain stage kernel. Shared memory is dynamic (a 32 x 32 tile needs

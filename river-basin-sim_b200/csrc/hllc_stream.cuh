@@ -44,125 +44,6 @@ __device__ __forceinline__ Quad east_of(const Quad& q) {
   return Quad{east_of(q.e), east_of(q.z), east_of(q.n), east_of(q.t)};
 }
 
-// The streaming kernel's forms of the cell and face arithmetic. Fast build: the formulas of
-// the functions above with the approximate units' flush-to-zero forms. Exact build: the
-// same values as the functions above without branches, by correctly rounded divisions and
-// square roots inside a safe range (rcp_rn, div_rn, sqrt_rn); `odd` is set where an
-// operand leaves it, and the caller redoes those lanes with the function above.
-#if defined(RB_FAST_MATH)
-__device__ __forceinline__ void primitives_near(float h, float hu, float hv, float& u, float& v, bool&) {
-  const bool wet = h > kHDry;
-  const float r = rcp_near(wet ? h : 1.0f);
-  u = wet ? hu * r : 0.0f;
-  v = wet ? hv * r : 0.0f;
-}
-
-__device__ __forceinline__ void hllc_near(float hl, float ul, float vtl, float hr, float ur, float vtr, float& f0,
-                                          float& f1, float& f2, bool&) {
-  const float g = kG;
-  const float cl = sqrt_near(g * fmaxf(hl, 0.0f)), cr = sqrt_near(g * fmaxf(hr, 0.0f));
-  const bool dry_l = hl <= kHDry, dry_r = hr <= kHDry;
-  const float c_star = fabsf(0.5f * (cl + cr) + 0.25f * (ul - ur));
-  const float u_star = 0.5f * (ul + ur) + cl - cr;
-  float sl = fminf(ul - cl, u_star - c_star), sr = fmaxf(ur + cr, u_star + c_star);
-  if (dry_r) sl = ul - cl, sr = ul + 2.0f * cl;
-  if (dry_l) sl = ur - 2.0f * cr, sr = ur + cr;
-  const float fh_l = hl * ul, fmn_l = hl * ul * ul + 0.5f * g * hl * hl;
-  const float fh_r = hr * ur, fmn_r = hr * ur * ur + 0.5f * g * hr * hr;
-  const float a = fminf(sl, 0.0f), b = fmaxf(sr, 0.0f);
-  const float inv = rcp_near(fmaxf(b - a, 1.0e-30f));
-  const float fh = (b * fh_l - a * fh_r + a * b * (hr - hl)) * inv;
-  const float fmn = (b * fmn_l - a * fmn_r + a * b * (hr * ur - hl * ul)) * inv;
-  const float den_s = hr * (ur - sr) - hl * (ul - sl);
-  const bool star_nonneg =
-      fabsf(den_s) > 1.0e-12f ? (sl * hr * (ur - sr) - sr * hl * (ul - sl)) * den_s >= 0.0f : ul + ur >= 0.0f;
-  const bool none = dry_l && dry_r;
-  f0 = none ? 0.0f : fh;
-  f1 = none ? 0.0f : fmn;
-  f2 = none ? 0.0f : fh * (star_nonneg ? vtl : vtr);
-}
-
-__device__ __forceinline__ void friction_near(float hh, bool wet, float gdt, float n, float& hu, float& hv) {
-  const float f = gdt * n * n * sqrt_near(hu * hu + hv * hv);
-  const float rd = rcp_near(1.0f + f * rcp_near(pow73_near(hh)));
-  if (wet) hu *= rd, hv *= rd;
-}
-
-__device__ __forceinline__ float wave_speed_near(float hh, float hu, float hv) {
-  const float cw = sqrt_near(kG * fmaxf(hh, 0.0f));
-  const bool wet = hh > kHDry;
-  return wet ? rmax(fabsf(hu), fabsf(hv)) * rcp_near(wet ? hh : 1.0f) + cw : cw;
-}
-#else
-__device__ __forceinline__ void primitives_near(float h, float hu, float hv, float& u, float& v, bool& odd) {
-  const bool wet = h > kHDry;
-  const float hs = wet ? h : 1.0f, y = rcp_rn(hs);
-  const float qu = div_rn_by(hu, hs, y), qv = div_rn_by(hv, hs, y);
-  u = wet ? qu : 0.0f;
-  v = wet ? qv : 0.0f;
-  const float m = fmaxf(fabsf(hu), fabsf(hv));
-  odd |= wet & !(div_rn_small_ok(hu) & div_rn_small_ok(hv) & (h <= 0x1p24f) & (m <= 0x1p60f));
-}
-
-__device__ __forceinline__ void hllc_near(float hl, float ul, float vtl, float hr, float ur, float vtr, float& f0,
-                                          float& f1, float& f2, bool& odd) {
-  const float g = kG;
-  const bool dry_l = hl <= kHDry, dry_r = hr <= kHDry, none = dry_l & dry_r;
-  // a dry side's celerity is not used
-  const float cl = sqrt_rn(g * (dry_l ? 1.0f : hl)), cr = sqrt_rn(g * (dry_r ? 1.0f : hr));
-  const float hs = 0.5f * (cl + cr) + 0.25f * (ul - ur);
-  const float hs2 = hs * hs;
-  const float c_star = sqrt_rn(g * rb_div_g_mid(hs2));
-  const float u_star = 0.5f * (ul + ur) + cl - cr;
-  float sl = rmin(ul - cl, u_star - c_star), sr = rmax(ur + cr, u_star + c_star);
-  if (dry_r) sl = ul - cl, sr = ul + 2.0f * cl;
-  if (dry_l) sl = ur - 2.0f * cr, sr = ur + cr;
-  const float fh_l = hl * ul, fmn_l = hl * ul * ul + 0.5f * g * hl * hl;
-  const float fh_r = hr * ur, fmn_r = hr * ur * ur + 0.5f * g * hr * hr;
-  const float gap = sr - sl, inv = rcp_rn(gap);
-  const float fh_m = (sr * fh_l - sl * fh_r + sl * sr * (hr - hl)) * inv;
-  const float fmn_m = (sr * fmn_l - sl * fmn_r + sl * sr * (hr * ur - hl * ul)) * inv;
-  const float fh = sl >= 0.0f ? fh_l : (sr <= 0.0f ? fh_r : fh_m);
-  const float fmn = sl >= 0.0f ? fmn_l : (sr <= 0.0f ? fmn_r : fmn_m);
-  // the sign of the contact speed num_s / den_s (quotient_nonneg without its rare cases)
-  const float den_s = hr * (ur - sr) - hl * (ul - sl);
-  const float num_s = sl * hr * (ur - sr) - sr * hl * (ul - sl);
-  const bool have_s = fabsf(den_s) > 1.0e-12f;
-  const bool nonneg = have_s ? (num_s == 0.0f) | ((num_s > 0.0f) == (den_s > 0.0f)) : 0.5f * (ul + ur) >= 0.0f;
-  const bool sign_ok = !have_s | (num_s == 0.0f) | (fabsf(num_s) > fabsf(den_s) * 0x1p-100f);
-  f0 = none ? 0.0f : fh;
-  f1 = none ? 0.0f : fmn;
-  f2 = none ? 0.0f : fh * (nonneg ? vtl : vtr);
-  odd |= !none & !((gap >= 0x1p-20f) & (gap <= 0x1p50f) & (dry_l | dry_r | (hs2 >= 0x1p-99f)) & sign_ok);
-}
-
-__device__ __forceinline__ void friction_near(float hh, bool wet, float gdt, float n, float& hu, float& hv) {
-  const float m2 = hu * hu + hv * hv, k = gdt * n * n;
-  const bool need = wet & !(((k == 0.0f) & (m2 <= FLT_MAX)) | ((m2 == 0.0f) & (k <= FLT_MAX)));
-  if (!__any_sync(kFullWarp, need)) return;
-  const float f = k * sqrt_rn(need ? m2 : 1.0f);
-  const float den = 1.0f + div_rn(f, pow73_mid(need ? hh : 1.0f));
-  const float y = rcp_rn(den);
-  const float qu = div_rn_by(hu, den, y), qv = div_rn_by(hv, den, y);
-  const bool ok = (m2 >= 0x1p-100f) & (m2 <= 0x1p100f) & (hh <= 0x1p19f) & (f <= 0x1p40f) & (den <= 0x1p20f) &
-                  div_rn_small_ok(hu) & div_rn_small_ok(hv);
-  if (__any_sync(kFullWarp, need & !ok))
-    hllc_friction(hh, wet, gdt, n, hu, hv);
-  else if (need)
-    hu = qu, hv = qv;
-}
-
-// The larger quotient is the larger dividend's: rounding is monotonic.
-__device__ __forceinline__ float wave_speed_near(float hh, float hu, float hv) {
-  const bool wet = hh > kHDry;
-  const float a = rmax(fabsf(hu), fabsf(hv)), hs = wet ? hh : 1.0f;
-  const bool ok = !wet | ((hh <= 0x1p24f) & (a <= 0x1p60f) & div_rn_small_ok(a));
-  if (__any_sync(kFullWarp, !ok | ((hh > 0.0f) & !(hh >= 0x1p-100f)))) return wave_speed(hh, hu, hv);
-  const float cw = hh > 0.0f ? sqrt_rn(kG * hh) : 0.0f;
-  return wet ? div_rn(a, hs) + cw : cw;
-}
-#endif
-
 // any_face_flux's operands for the face: what goes into the Riemann solve (the ghost
 // states of an edge face included) and the depths of the bed-slope corrections.
 struct FaceOperands {
@@ -345,7 +226,7 @@ __device__ __forceinline__ void hllc_stream_strip(const HllcParams& p, const Hll
     bool odd0 = false;
     primitives_near(h0, now[32], now[64], u0, v0, odd0);
 #if !defined(RB_FAST_MATH)
-    if (__any_sync(kFullWarp, odd0)) primitives(h0, now[32], now[64], u0, v0);
+    if (__any_sync(kFullWarp, odd0)) primitives_any(h0, now[32], now[64], u0, v0);
 #endif
     const Quad c0q{h0 + z0, z0, v0, u0};  // the y frame: normal v, transverse u
     const Quad d0 = c0q - c1;
@@ -383,8 +264,8 @@ __device__ __forceinline__ void hllc_stream_strip(const HllcParams& p, const Hll
       hllc_near(ox.hl, ox.ul, ox.vl, ox.hr, ox.ur, ox.vr, x0, x1f, x2, odd);
 #if !defined(RB_FAST_MATH)
       if (__any_sync(kFullWarp, odd)) {
-        hllc_flux(oy.hl, oy.ul, oy.vl, oy.hr, oy.ur, oy.vr, y0, y1, y2);
-        hllc_flux(ox.hl, ox.ul, ox.vl, ox.hr, ox.ur, ox.vr, x0, x1f, x2);
+        hllc_flux_any(oy.hl, oy.ul, oy.vl, oy.hr, oy.ur, oy.vr, y0, y1, y2);
+        hllc_flux_any(ox.hl, ox.ul, ox.vl, ox.hr, ox.ur, ox.vr, x0, x1f, x2);
       }
 #endif
       fy = face_flux(oy, y0, y1, y2, kind_y, fi == 0);
@@ -441,7 +322,7 @@ __device__ __forceinline__ void hllc_stream_strip(const HllcParams& p, const Hll
         const bool wet = hh > kHDry;
         float hu = wet ? 0.5f * (now[(Ring::kOld + 1) * 32] + hus + dt * dhu3) : 0.0f;
         float hv = wet ? 0.5f * (now[(Ring::kOld + 2) * 32] + hvs + dt * dhv3) : 0.0f;
-        friction_near(hh, wet, g * dt, now[(Ring::kOld + 3) * 32], hu, hv);
+        hllc_friction<true>(hh, wet, g * dt, now[(Ring::kOld + 3) * 32], hu, hv);
         if (SRC != 0 && s.rain_mode == 1) {
           float comp = now[Ring::kSrc * 32];
           kahan_add(hh, comp, s.rain32 * dt);
@@ -472,7 +353,7 @@ __device__ __forceinline__ void hllc_stream_strip(const HllcParams& p, const Hll
           hu_out[id3] = hu;
           hv_out[id3] = hv;
         }
-        const float sp = wave_speed_near(hh, hu, hv);  // hllc.py:948-966 on the new state
+        const float sp = wave_speed<true>(hh, hu, hv);  // hllc.py:948-966 on the new state
         smax = fmaxf(smax, EDGE && !own ? 0.0f : sp);
         bad |= (!EDGE | own) & (!(fabsf(hh) <= FLT_MAX) | !(fabsf(hu) <= FLT_MAX) | !(fabsf(hv) <= FLT_MAX));
       }

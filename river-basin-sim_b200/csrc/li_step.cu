@@ -41,6 +41,8 @@
 namespace rb {
 RB_ARITH_BEGIN
 
+#include "warp_stream.cuh"
+
 #if defined(RB_FAST_MATH)
 constexpr bool kEarlySedLoads = true;
 #else
@@ -190,7 +192,7 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
   float* __restrict__ h_out = p.hb[cur ^ 1];
   float* __restrict__ qx_out = p.qxb[cur ^ 1];
   float* __restrict__ qy_out = p.qyb[cur ^ 1];
-  const float dx = p.dx32;
+  const float dx = p.dx32, rdx = slope_rcp(dx);
   const float dtdx = dt / dx;
 
   // 1. stage h, z, n (halo 2) and eta = h + z (local_inertial.py:61-69), and the
@@ -318,7 +320,7 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
             if (!(h_flow < kHDry)) {
               const float qo = s_qx[a][b];  // previous discharge, staged above
               const float n_face = 0.5f * (s_n[a + 1][b] + s_n[a + 1][b + 1]);
-              const float slope = div_pos(eta_r - eta_l, dx);
+              const float slope = face_slope(eta_r - eta_l, dx, rdx);
               const float num = qo - kG * h_flow * dt * slope;
               q = manning_divide(num, qo, h_flow, n_face, kG, dt);
             }
@@ -329,7 +331,7 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
             const int r = a + 1, cl = b, cr = b + 1;
             const float eta_l = s_eta[r][cl], eta_r = s_eta[r][cr];
             const float eta_max = rmax(eta_l, eta_r);
-            const float slope = div_pos(eta_r - eta_l, dx);
+            const float slope = face_slope(eta_r - eta_l, dx, rdx);
             const float z_bank = rmax(s_z[r][cl], s_z[r][cr]);
             qf = floodplain_flux(S.ch.qxf[a][b], eta_max, slope, z_bank, 0.5f * (s_n[r][cl] + s_n[r][cr]), dt);
             const float w_face = rmin(S.ch.w[r][cl], S.ch.w[r][cr]);
@@ -355,7 +357,7 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
             if (!(h_flow < kHDry)) {
               const float qo = s_qy[a][b];
               const float n_face = 0.5f * (s_n[a][b + 1] + s_n[a + 1][b + 1]);
-              const float slope = div_pos(eta_b - eta_t, dx);
+              const float slope = face_slope(eta_b - eta_t, dx, rdx);
               const float num = qo - kG * h_flow * dt * slope;
               q = manning_divide(num, qo, h_flow, n_face, kG, dt);
             }
@@ -366,7 +368,7 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
             const int c = b + 1, rt = a, rb = a + 1;
             const float eta_t = s_eta[rt][c], eta_b = s_eta[rb][c];
             const float eta_max = rmax(eta_t, eta_b);
-            const float slope = div_pos(eta_b - eta_t, dx);
+            const float slope = face_slope(eta_b - eta_t, dx, rdx);
             const float z_bank = rmax(s_z[rt][c], s_z[rb][c]);
             qf = floodplain_flux(S.ch.qyf[a][b], eta_max, slope, z_bank, 0.5f * (s_n[rt][c] + s_n[rb][c]), dt);
             const float w_face = rmin(S.ch.w[rt][c], S.ch.w[rb][c]);
@@ -395,19 +397,12 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
   if (limit) {
     for (int k = threadIdx.x; k < BH * BW; k += NT) {
       const int a = k / BW, b = k - a * BW;
-      float q_out = 0.0f;
-      const float ql = s_qx[a][b];
-      if (ql < 0.0f) q_out = q_out - ql;
-      const float qr = s_qx[a][b + 1];
-      if (qr > 0.0f) q_out = q_out + qr;
-      const float qt = s_qy[a][b];
-      if (qt < 0.0f) q_out = q_out - qt;
-      const float qb = s_qy[a + 1][b];
-      if (qb > 0.0f) q_out = q_out + qb;
-      const float out_depth = dtdx * q_out;
-      const bool out = out_depth > 0.0f;
-      const float ratio = div_if(out, s_h[a + 1][b + 1], out_depth);
-      s_beta[a][b] = out ? rclamp(ratio, 0.0f, 1.0f) : 1.0f;
+      const float q_out =
+          fmaxf(-s_qx[a][b], 0.0f) + fmaxf(s_qx[a][b + 1], 0.0f) + fmaxf(-s_qy[a][b], 0.0f) + fmaxf(s_qy[a + 1][b], 0.0f);
+      const float out_depth = dtdx * q_out, hc = s_h[a + 1][b + 1];
+      float beta = 1.0f;  // h >= out_depth gives 1
+      if (out_depth > 0.0f && !(hc >= out_depth)) beta = rclamp(div_in_branch(hc, out_depth), 0.0f, 1.0f);
+      s_beta[a][b] = beta;
     }
     __syncthreads();
   }
@@ -658,7 +653,6 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
   __syncthreads();  // the shared tile is reused by the caller's next tile
 }
 
-#include "warp_stream.cuh"
 #include "li_stream.cuh"
 
 // The single-domain step kernel. MINB is __launch_bounds__' resident-block hint (it

@@ -37,8 +37,7 @@ __device__ __forceinline__ void li_faces(const float (&qo)[NF], const float (&el
   for (int i = 0; i < NF; i++) {
     const float slope = (er[i] - el[i]) * c.rdx;
     const float num = qo[i] - kG * h[i] * c.dt * slope;
-    const float f = c.gdt * n[i] * n[i] * fabsf(qo[i]);
-    const float v = num * rcp_near(1.0f + f * rcp_near(pow73_near(h[i])));
+    const float v = manning_divide(num, qo[i], h[i], n[i], kG, c.dt);
     q[i] = !on[i] || h[i] < kHDry ? 0.0f : v;
   }
 }
@@ -84,7 +83,8 @@ __device__ __forceinline__ void li_faces(const float (&qo)[NF], const float (&el
       for (int j = 0; j < NF; j++) {
         if (j == i) o = qo[j], l = el[j], r = er[j], hh = h[j], nn = n[j], w = wet[j];
       }
-      if (w) qi = manning_divide(o - kG * hh * c.dt * div_pos(r - l, c.dx), o, hh, nn, kG, c.dt);
+      if (w)
+        qi = manning_divide_any(o - kG * hh * c.dt * div_pos(r - l, c.dx), c.gdt * nn * nn * fabsf(o), hh);
 #pragma unroll
       for (int j = 0; j < NF; j++) {
         if (j == i) q[j] = qi;
@@ -98,12 +98,7 @@ __device__ __forceinline__ LiFaceConst li_face_const(float dt, float dx) {
   LiFaceConst c;
   c.dt = dt;
   c.dx = dx;
-#if defined(RB_FAST_MATH)
-  c.rdx = rcp_near(dx);
-#else
-  // 0 where dx is outside div_rn's range: every face then takes the divisions
-  c.rdx = dx >= 0x1p-20f && dx <= 0x1p20f ? 1.0f / dx : 0.0f;
-#endif
+  c.rdx = slope_rcp(dx);
   c.gdt = kG * dt;
   return c;
 }

@@ -233,14 +233,51 @@ __device__ __forceinline__ float manning_denominator(float q_prev, float h_flow,
   return 1.0f + g * dt * n * n * fabsf(q_prev) / pow73(h_flow);
 }
 
-// num / manning_denominator(q_prev, h_flow, n, g, dt) for h_flow >= H_DRY, with the
-// same bits: when the friction numerator g dt n^2 |q_prev| is +0 the denominator is
-// exactly 1 (and num / 1 == num), so neither the power nor the divisions are needed.
+// num / manning_denominator(q_prev, h_flow, n, g, dt) for h_flow >= H_DRY, with the same
+// bits. Where the friction numerator f = g dt n^2 |q_prev| is +0 or below 2^-60 the
+// denominator is exactly 1 (h^(7/3) > 2^-24) and the quotient the numerator.
+#if defined(RB_FAST_MATH)
 __device__ __forceinline__ float manning_divide(float num, float q_prev, float h_flow, float n, float g, float dt) {
   const float f = g * dt * n * n * fabsf(q_prev);
+  return num * rcp_near(1.0f + f * rcp_near(pow73_near(h_flow)));
+}
+#else
+__device__ __forceinline__ float manning_divide_any(float num, float f, float h_flow) {
   if (f == 0.0f) return num;
-  const float den = 1.0f + f / pow73(h_flow);
-  return div_pos(num, den);
+  return div_pos(num, 1.0f + f / pow73(h_flow));
+}
+// The quick divisions and power inside their ranges, the general ones outside.
+__device__ __forceinline__ float manning_divide(float num, float q_prev, float h_flow, float n, float g, float dt) {
+  const float f = g * dt * n * n * fabsf(q_prev);
+  float q = num;
+  if (!(f < 0x1p-60f)) {
+    const float den = 1.0f + div_rn(f, pow73_mid(h_flow));
+    q = div_rn(num, den);
+    const bool ok = (h_flow <= 0x1p19f) & (f <= 0x1p40f) & (den <= 0x1p20f) & div_rn_small_ok(num) &
+                    !(fabsf(num) > 0x1p60f);
+    if (!ok) q = manning_divide_any(num, f, h_flow);
+  }
+  return q;
+}
+#endif
+
+// The reciprocal of dx a kernel's surface slopes multiply by, 0 where it must divide.
+__device__ __forceinline__ float slope_rcp(float dx) {
+#if defined(RB_FAST_MATH)
+  return rcp_near(dx);
+#else
+  return dx >= 0x1p-20f && dx <= 0x1p20f ? 1.0f / dx : 0.0f;
+#endif
+}
+// de / dx with rdx = slope_rcp(dx), the same bits.
+__device__ __forceinline__ float face_slope(float de, float dx, float rdx) {
+#if defined(RB_FAST_MATH)
+  return de * rdx;
+#else
+  const float q = div_rn_by(de, dx, rdx);
+  if (rdx == 0.0f || !div_rn_small_ok(de) || fabsf(de) > 0x1p60f) return div_in_branch(de, dx);
+  return q;
+#endif
 }
 
 // Float key whose unsigned order is the float order for values >= 0.

@@ -5,6 +5,13 @@
 
 constexpr unsigned kFullWarp = 0xffffffffu;
 
+// Whether any lane of the warp has `p` (VOTE: all of its lanes call), or this one.
+template <bool VOTE>
+__device__ __forceinline__ bool any_lane(bool p) {
+  if constexpr (VOTE) return __any_sync(kFullWarp, p);
+  return p;
+}
+
 // The value one cell to the west / east of this lane's (the outermost lanes get their own
 // back: they hold halo cells whose results nobody stores).
 __device__ __forceinline__ float west_of(float x) { return __shfl_up_sync(kFullWarp, x, 1); }
