@@ -443,17 +443,17 @@ static cudaError_t launch_hllc_stream(const HllcParams& p, int stage, cudaStream
              : launch_chain(hllc_stream_kernel<2, 0>, grid, block, 0, s, p, rows);
 }
 
-// Whether the streaming kernel takes this domain (with hllc_stream_fits). Below this many
-// cells the 32 x 32 tiles are as fast or faster: a warp walks its rows one after another,
-// and a small domain has too few warps to hide that (dam breaks, us per step, tiles /
-// streaming -- fast: 700^2 44 / 50, 1024^2 72.0 / 73.8, 1448^2 138 / 114, 2048^2 265 / 190,
-// 4096^2 1011 / 633; exact: 1024^2 88 / 99, 1448^2 169 / 162, 2048^2 325 / 268, 4096^2
-// 1244 / 912).
+// Whether the streaming kernel takes this domain (with hllc_stream_fits). Below these sizes
+// the 32 x 32 tiles are as fast or faster: a warp walks its rows one after another, and a
+// small domain has too few warps to hide that; on a narrow one the strips at the west and
+// east edge, which check bounds, are too many (dam breaks, us per step, tiles / streaming
+// -- fast: 1024^2 72.0 / 73.8, 1448^2 138 / 114, 2048^2 265 / 190, 4096^2 1011 / 633; exact:
+// 1448^2 161 / 162, 2048^2 306 / 268, 4096^2 1180 / 912; lake, 2600 x 480 fast 91.7 / 98.7).
 #if defined(RB_FAST_MATH)
-constexpr long long kHllcStreamCells = 1200000;
+constexpr long long kHllcStreamCells = 1500000;
 #else
-constexpr long long kHllcStreamCells = 2000000;
+constexpr long long kHllcStreamCells = 3000000;
 #endif
 static bool hllc_stream_takes(const HllcParams& p) {
-  return (long long)p.ny * p.nx >= kHllcStreamCells && hllc_stream_fits(p.ny, p.nx);
+  return (long long)p.ny * p.nx >= kHllcStreamCells && p.nx >= 30 * kHllcStreamCols && hllc_stream_fits(p.ny, p.nx);
 }
