@@ -146,7 +146,8 @@ __device__ void clock_plan(DevClock* c) {
 }
 
 __global__ void clock_plan_kernel(DevClock* c) {
-  pdl_enter();
+  pdl_trigger();
+  pdl_wait();
   clock_plan(c);
 }
 

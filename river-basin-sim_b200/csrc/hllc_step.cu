@@ -1067,6 +1067,7 @@ __device__ __forceinline__ bool hllc_tile(const HllcParams& p, int bx, int by, s
     }
   }
 
+  pdl_trigger();
   // An interior tile banks nothing but infiltration (it has no edge face), so without
   // infiltration its loss is 0 and its slot, zero from the start, stays exactly 0:
   // the block sum is skipped.
@@ -1093,7 +1094,7 @@ __global__ void __launch_bounds__(NT, NT > 512 ? 2 : 1024 / NT) hllc_stage_kerne
   extern __shared__ __align__(16) unsigned char hllc_smem_raw[];
   using SMEM = typename HllcSmemOf<TX, TY, FU, LP>::type;
   auto& S = *reinterpret_cast<SMEM*>(hllc_smem_raw);
-  pdl_enter();
+  pdl_wait();
   const size_t slot = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
   if (hllc_deep_interior<TX, TY>(blockIdx.x * TX, blockIdx.y * TY, p.ny, p.nx))
     hllc_tile<TX, TY, NT, STAGE, FU, LP, true, SRC>(p, blockIdx.x, blockIdx.y, slot, S);
@@ -1141,7 +1142,7 @@ __global__ void __launch_bounds__(NT, NT > 512 ? 2 : 1024 / NT)
     hllc_stage_tma_kernel(const HllcParams p, const __grid_constant__ HllcMaps maps) {
   extern __shared__ __align__(1024) unsigned char hllc_tma_smem_raw[];
   auto& S = *reinterpret_cast<HllcSmemTma<TX, TY>*>(hllc_tma_smem_raw);
-  pdl_enter();
+  pdl_wait();
   const size_t slot = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
   if (hllc_deep_interior<TX, TY>(blockIdx.x * TX, blockIdx.y * TY, p.ny, p.nx))
     hllc_tile<TX, TY, NT, STAGE, 1, 2, true>(p, blockIdx.x, blockIdx.y, slot, S, &maps);
@@ -1158,7 +1159,7 @@ __global__ void __launch_bounds__(NT, NT > 512 ? 2 : 1024 / NT)
     hllc_stage_tma_pipe_kernel(const HllcParams p, const __grid_constant__ HllcMaps maps) {
   extern __shared__ __align__(1024) unsigned char hllc_pipe_smem_raw[];
   auto& S = *reinterpret_cast<HllcSmemTma<TX, TY>*>(hllc_pipe_smem_raw);
-  pdl_enter();
+  pdl_wait();
   if (p.clk != nullptr && !p.clk->active) return;  // no tile works this step
   const int cur = p.clk != nullptr ? p.clk->cur : p.cur;
   if (threadIdx.x == 0) {

@@ -405,7 +405,7 @@ constexpr int kHllcStreamWarps = 16;
 template <int STAGE, int SRC>
 __global__ void __launch_bounds__(32, kHllcStreamWarps) hllc_stream_kernel(const HllcParams p, int rows) {
   __shared__ HllcRing<STAGE, SRC> ring;
-  pdl_enter();
+  pdl_wait();
   HllcStageScalars s;
   if (!hllc_scalars(p, s)) return;
   const int c0 = blockIdx.x * kHllcStreamCols - kHllcHalo;
@@ -420,6 +420,7 @@ __global__ void __launch_bounds__(32, kHllcStreamWarps) hllc_stream_kernel(const
     hllc_stream_strip<STAGE, SRC, false>(p, s, c0, i0, i1, ring, loss, smax, bad);
   else
     hllc_stream_strip<STAGE, SRC, true>(p, s, c0, i0, i1, ring, loss, smax, bad);
+  pdl_trigger();
   const int lane = threadIdx.x;
   if (p.ledger != nullptr) {
     const double t = warp_sum(loss);

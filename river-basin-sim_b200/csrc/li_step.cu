@@ -641,6 +641,7 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
     bad |= !(fabsf(h) <= FLT_MAX);
   }
 
+  pdl_trigger();
   // An interior tile banks nothing but infiltration (no cell of it drains through an
   // edge), so without infiltration its loss is 0 and its slot, zero from the start,
   // stays exactly 0: the block sum is skipped.
@@ -660,7 +661,7 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
 template <int TX, int TY, int NT, bool CH, int MINB, int SED>
 __global__ void __launch_bounds__(NT, MINB) li_step_kernel(const LiParams p) {
   __shared__ LiSmem<TX, TY, CH> S;
-  pdl_enter();
+  pdl_wait();
   const size_t slot = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
   if (li_deep_interior<TX, TY>(blockIdx.x * TX, blockIdx.y * TY, p.ny, p.nx))
     li_tile<TX, TY, NT, CH, true, SED>(p, blockIdx.x, blockIdx.y, slot, S);

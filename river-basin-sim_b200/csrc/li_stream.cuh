@@ -377,7 +377,7 @@ __device__ __forceinline__ void li_stream_strip(const LiParams& p, const LiStepS
 template <int SED, int SRC>
 __global__ void __launch_bounds__(32, kLiStreamWarps) li_stream_kernel(const LiParams p, int rows) {
   __shared__ LiRing<SED, SRC> ring;
-  pdl_enter();
+  pdl_wait();
   LiStepScalars s;
   if (!li_scalars(p, s)) return;
   const int c0 = blockIdx.x * kLiStreamCols - kLiHalo;
@@ -392,6 +392,7 @@ __global__ void __launch_bounds__(32, kLiStreamWarps) li_stream_kernel(const LiP
     li_stream_strip<SED, SRC, false>(p, s, c0, i0, i1, ring, loss, hmax, bad);
   else
     li_stream_strip<SED, SRC, true>(p, s, c0, i0, i1, ring, loss, hmax, bad);
+  pdl_trigger();
   const int lane = threadIdx.x;
   if (p.ledger != nullptr) {
     const double t = warp_sum(loss);
