@@ -1358,6 +1358,8 @@ void hllc_prepare_device() {
   prepare_hllc<32, 32, 512, 1, 1>();
   prepare_hllc<64, 16, 512, 1, 1>();
   prepare_hllc<32, 32, 640, 1, 1>();
+  prepare_hllc<16, 16, 704, 1, 1>();
+  prepare_hllc<32, 16, 640, 1, 1>();
   prepare_hllc_tma<32, 32, 640>();
   hllc_pipe_grid<32, 32, 512>();
 #if !defined(RB_FAST_MATH)
@@ -1398,8 +1400,13 @@ cudaError_t hllc_stage_launch_exact(const HllcParams& p, int stage, int variant,
     case 4: return launch_hllc<32, 32, 512, 1, 1>(p, stage, s);
     case 7: return launch_hllc_tma<32, 32, 640>(p, stage, s);
     case 8: return launch_hllc_tma<32, 32, 512, true>(p, stage, s);
-    default:
-      return hllc_stream_takes(p) ? launch_hllc_stream(p, stage, s) : launch_hllc<32, 32, 640, 1, 1>(p, stage, s);
+    default: break;
+  }
+  if (hllc_stream_takes(p)) return launch_hllc_stream(p, stage, s);
+  switch (hllc_default_tile(p.ny, p.nx)) {
+    case 0: return launch_hllc<16, 16, 704, 1, 1>(p, stage, s);
+    case 1: return launch_hllc<32, 16, 640, 1, 1>(p, stage, s);
+    default: return launch_hllc<32, 32, 640, 1, 1>(p, stage, s);
   }
 }
 
@@ -1411,10 +1418,16 @@ int hllc_tiles(int ny, int nx) { return hllc_tiles_of(g_hllc_variant.load(), ny,
 int hllc_tiles_of(int variant, int ny, int nx) {
   const bool known = variant >= 0 && variant < kNumHllcVariants;
   const HllcKernelVariant& v = kHllcVariants[known ? variant : kDefaultHllcVariant];
-  const int tiles = ((nx + v.tx - 1) / v.tx) * ((ny + v.ty - 1) / v.ty);
-  // the default variant's streaming kernel, in either arithmetic, has a slot per block
-  const bool stream = (!known || variant == kDefaultHllcVariant) && hllc_stream_fits(ny, nx);
-  return stream ? std::max(tiles, hllc_stream_blocks(ny, nx)) : tiles;
+  int tx = v.tx, ty = v.ty;
+  const bool by_size = !known || variant == kDefaultHllcVariant;
+  if (by_size) {  // the default variant chooses its tile by the domain's size
+    const int t = hllc_default_tile(ny, nx);
+    tx = t == 0 ? 16 : 32;
+    ty = t <= 1 ? 16 : 32;
+  }
+  const int tiles = ((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
+  // its streaming kernel, in either arithmetic, has a slot per block
+  return by_size && hllc_stream_fits(ny, nx) ? std::max(tiles, hllc_stream_blocks(ny, nx)) : tiles;
 }
 
 // Ensemble: one Heun stage over the (domain, local tile) work-list of every HLLC

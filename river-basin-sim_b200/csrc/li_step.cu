@@ -678,6 +678,17 @@ static cudaError_t launch_li(const LiParams& p, cudaStream_t s) {
                           : launch_chain(li_step_kernel<TX, TY, NT, CH, MINB, 0>, grid, dim3(NT), 0, s, p);
 }
 
+// A domain of few 32 x 32 tiles leaves most SMs idle and its step is one tile's latency:
+// 16 x 16 tiles with as many threads spread it over four times the SMs and halve the
+// passes of a block (rain-on-grid, us per clocked step, 32 x 32 / 16 x 16: 128^2 12.9 / 9.7,
+// 256^2 14.7 / 11.7, 400^2 14.8 / 16.9). The ledger has a slot per 32 x 8 cells, too few
+// for 16 x 16 tiles on some narrow domains.
+constexpr long long kLiSmallCells = 100000;
+static bool li_small(const LiParams& p) {
+  const long long tiles = (long long)((p.nx + 15) / 16) * ((p.ny + 15) / 16);
+  return (long long)p.ny * p.nx <= kLiSmallCells && tiles <= (long long)((p.nx + 31) / 32) * ((p.ny + 7) / 8);
+}
+
 // Tile variants of the single-domain step (sub-grid channels always use 32 x 16);
 // all compute the same bits. The default is the fastest measured on B200 for the
 // 2048^2 and 4096^2 rain-on-grid steps (ms per 2048^2 step: 0.158, 0.142, 0.145,
@@ -713,8 +724,10 @@ cudaError_t li_step_launch_variant(const LiParams& p, int variant, cudaStream_t 
     case 2: return launch_li<64, 16, 512, false, 3>(p, s);
     case 3: return launch_li<32, 8, 256, false, 1>(p, s);
     case 4: return launch_li<32, 16, 256, false, 5>(p, s);  // at most 48 registers
-    default: return li_stream_takes(p) ? launch_li_stream(p, s) : launch_li<32, 32, 512, false, 3>(p, s);
+    default: break;
   }
+  if (li_stream_takes(p)) return launch_li_stream(p, s);
+  return li_small(p) ? launch_li<16, 16, 512, false, 2>(p, s) : launch_li<32, 32, 512, false, 3>(p, s);
 }
 
 #if !defined(RB_FAST_MATH)

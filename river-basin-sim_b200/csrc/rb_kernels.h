@@ -119,6 +119,19 @@ inline bool hllc_stream_fits(int ny, int nx) {
          (long long)(rows + 16) * nx < (1LL << 31);
 }
 
+// The tile of the default HLLC variant below the streaming kernel's sizes: 0 = 16 x 16
+// (704 threads, one pass over its 684 faces), 1 = 32 x 16, 2 = 32 x 32 (640 threads). Few
+// large tiles leave most SMs idle and a stage is one tile's latency (dam break, us per
+// clocked step, 16 x 16 / 32 x 16 / 32 x 32: 128^2 13.2 / 15.5 / 22.3, 256^2 17.4 / 17.3 /
+// 22.1, 400^2 29.9 / 28.0 / 30.7, 512^2 38.7 / 33.8 / 32.2). The ledger has a slot per 32 x
+// 8 cells, too few for 16 x 16 tiles on some narrow domains.
+inline int hllc_default_tile(int ny, int nx) {
+  const long long cells = (long long)ny * nx;
+  const long long t16 = (long long)((nx + 15) / 16) * ((ny + 15) / 16);
+  if (cells <= 75000 && t16 <= (long long)((nx + 31) / 32) * ((ny + 7) / 8)) return 0;
+  return cells <= 200000 ? 1 : 2;
+}
+
 // The tensor maps (CUtensorMap, 128 bytes each, held opaque here) of the fields the
 // TMA-staged HLLC stage kernel copies into shared memory: both buffers of h, hu, hv
 // (the clock picks one at run time), the bed and the stage-1 state.
