@@ -8,67 +8,75 @@ namespace rb {
 
 constexpr int RED_NT = 256;
 
-// local_inertial.py:503-512 reduce_hmax: max(0, max h) into a zeroed slot.
-__global__ void __launch_bounds__(RED_NT) max_h_kernel(const float* __restrict__ h, size_t n, unsigned int* key) {
-  __shared__ float s_w[RED_NT / 32];
-  float m = 0.0f;
-  for (size_t k = (size_t)blockIdx.x * RED_NT + threadIdx.x; k < n; k += (size_t)gridDim.x * RED_NT) {
-    const float v = h[k];
-    m = v > m ? v : m;
-  }
-  block_max_to<RED_NT>(m, key, s_w);
-}
-
-// local_inertial.py:475-489 reduce_column_max into a zeroed slot.
-__global__ void __launch_bounds__(RED_NT) max_column_kernel(const float* __restrict__ h, const float* __restrict__ w,
-                                                             const float* __restrict__ d, float dx, size_t n,
-                                                             unsigned int* key) {
-  __shared__ float s_w[RED_NT / 32];
-  float m = 0.0f;
-  for (size_t k = (size_t)blockIdx.x * RED_NT + threadIdx.x; k < n; k += (size_t)gridDim.x * RED_NT) {
-    const float v = column_depth(h[k], w[k], d[k], dx);
-    m = v > m ? v : m;
-  }
-  block_max_to<RED_NT>(m, key, s_w);
-}
-
-// hllc.py:948-966 _reduce_wavespeed into a zeroed slot.
-__global__ void __launch_bounds__(RED_NT) wavespeed_kernel(const float* __restrict__ h, const float* __restrict__ hu,
-                                                            const float* __restrict__ hv, size_t n,
-                                                            unsigned int* key) {
-  __shared__ float s_w[RED_NT / 32];
-  float m = 0.0f;
-  for (size_t k = (size_t)blockIdx.x * RED_NT + threadIdx.x; k < n; k += (size_t)gridDim.x * RED_NT) {
+// The reductions of compute_dt: the largest of a non-negative per-cell value. One launch:
+// each block folds its maximum into the workspace's accumulator and the last one to finish
+// hands the result to `out` (a device word or a mapped host word) and clears the
+// accumulator and the ticket for the next call (calls on one workspace do not overlap).
+// It was two launches and a copy back: 97 x 161 compute_dt + step, 40.6 us a step.
+struct MaxH {  // local_inertial.py:503-512 reduce_hmax: max(0, max h)
+  const float* h;
+  __device__ float operator()(size_t k) const { return h[k]; }
+};
+struct MaxColumn {  // local_inertial.py:475-489 reduce_column_max
+  const float *h, *w, *d;
+  float dx;
+  __device__ float operator()(size_t k) const { return column_depth(h[k], w[k], d[k], dx); }
+};
+struct MaxSpeed {  // hllc.py:948-966 _reduce_wavespeed
+  const float *h, *hu, *hv;
+  __device__ float operator()(size_t k) const {
     const float hh = h[k];
     const float c = sqrtf(kG * rmax(hh, 0.0f));
     const bool wet = hh > kHDry;
-    const float s = wet ? rmax(div_if(wet, fabsf(hu[k]), hh), div_if(wet, fabsf(hv[k]), hh)) + c : c;
-    m = s > m ? s : m;
+    return wet ? rmax(div_if(wet, fabsf(hu[k]), hh), div_if(wet, fabsf(hv[k]), hh)) + c : c;
   }
-  block_max_to<RED_NT>(m, key, s_w);
+};
+
+constexpr int kMaxPerThread = 4;  // values in flight per thread and pass
+template <class F>
+__global__ void __launch_bounds__(RED_NT) max_kernel(const F f, size_t n, MaxScratch* scratch, unsigned int* out) {
+  __shared__ float s_w[RED_NT / 32];
+  float m = 0.0f;
+  const size_t step = (size_t)gridDim.x * RED_NT * kMaxPerThread;
+  for (size_t k = (size_t)blockIdx.x * RED_NT * kMaxPerThread + threadIdx.x; k < n; k += step) {
+    float v[kMaxPerThread];
+#pragma unroll
+    for (int i = 0; i < kMaxPerThread; i++) v[i] = k + (size_t)i * RED_NT < n ? f(k + (size_t)i * RED_NT) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < kMaxPerThread; i++) m = v[i] > m ? v[i] : m;
+  }
+  m = warp_max(m);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) s_w[w] = m;
+  __syncthreads();
+  if (w != 0) return;
+  m = warp_max(l < RED_NT / 32 ? s_w[l] : 0.0f);
+  if (l != 0) return;
+  atomicMax(&scratch->key, max_key(m));
+  __threadfence();
+  if (atomicAdd(&scratch->ticket, 1u) == gridDim.x - 1) {
+    __threadfence();
+    *out = atomicExch(&scratch->key, 0u);
+    scratch->ticket = 0u;
+  }
 }
 
-__global__ void zero_key_kernel(unsigned int* key) { *key = 0u; }
-
-cudaError_t reduce_max_h(const float* h, size_t n, unsigned int* key, cudaStream_t s) {
-  zero_key_kernel<<<1, 1, 0, s>>>(key);
-  max_h_kernel<<<WS_SUM_BLOCKS, RED_NT, 0, s>>>(h, n, key);
+template <class F>
+static cudaError_t reduce_max(const F& f, size_t n, MaxScratch* scratch, unsigned int* out, cudaStream_t s) {
+  const size_t blocks = (n + RED_NT * kMaxPerThread - 1) / (RED_NT * kMaxPerThread);
+  max_kernel<<<(unsigned)(blocks < WS_SUM_BLOCKS ? blocks : WS_SUM_BLOCKS), RED_NT, 0, s>>>(f, n, scratch, out);
   return cudaGetLastError();
 }
 
 cudaError_t reduce_max_column(const float* h, const float* w, const float* d, float dx32, size_t n,
-                              unsigned int* key, cudaStream_t s) {
-  if (w == nullptr) return reduce_max_h(h, n, key, s);
-  zero_key_kernel<<<1, 1, 0, s>>>(key);
-  max_column_kernel<<<WS_SUM_BLOCKS, RED_NT, 0, s>>>(h, w, d, dx32, n, key);
-  return cudaGetLastError();
+                              MaxScratch* scratch, unsigned int* out, cudaStream_t s) {
+  if (w == nullptr) return reduce_max(MaxH{h}, n, scratch, out, s);
+  return reduce_max(MaxColumn{h, w, d, dx32}, n, scratch, out, s);
 }
 
-cudaError_t reduce_wavespeed(const float* h, const float* hu, const float* hv, size_t n, unsigned int* key,
-                             cudaStream_t s) {
-  zero_key_kernel<<<1, 1, 0, s>>>(key);
-  wavespeed_kernel<<<WS_SUM_BLOCKS, RED_NT, 0, s>>>(h, hu, hv, n, key);
-  return cudaGetLastError();
+cudaError_t reduce_wavespeed(const float* h, const float* hu, const float* hv, size_t n, MaxScratch* scratch,
+                             unsigned int* out, cudaStream_t s) {
+  return reduce_max(MaxSpeed{h, hu, hv}, n, scratch, out, s);
 }
 
 // Deterministic float64 sum: a fixed grid of WS_SUM_BLOCKS blocks with a fixed

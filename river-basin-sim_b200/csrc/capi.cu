@@ -44,6 +44,48 @@ inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 rb::WsHeader* header(void* ws) { return static_cast<rb::WsHeader*>(ws); }
 
+// Where a reduction's one word comes back: a mapped, page-locked host word that the kernel
+// writes itself, one per host thread (given back when the thread ends), which saves the
+// copy's launch and its staging; or, where none can be had, the workspace's word and a copy.
+// The caller synchronises before it reads, so a thread has one in flight at most.
+struct MappedWord {
+  unsigned int* host = nullptr;
+  MappedWord() {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
+      host = static_cast<unsigned int*>(p);
+    else
+      cudaGetLastError();
+  }
+  ~MappedWord() {
+    if (host != nullptr) cudaFreeHost(host);
+  }
+};
+
+struct ResultWord {
+  unsigned int* device;
+  unsigned int* mapped = nullptr;
+  explicit ResultWord(rb::WsHeader* h) : device(&h->red_key) {
+    static thread_local MappedWord word;
+    void* d = nullptr;
+    if (word.host == nullptr) return;
+    if (cudaHostGetDevicePointer(&d, word.host, 0) == cudaSuccess) {
+      mapped = word.host;
+      device = static_cast<unsigned int*>(d);
+    } else {
+      cudaGetLastError();
+    }
+  }
+  int read(float* out, cudaStream_t s, const char* who) const {
+    unsigned int key = 0;
+    if (mapped == nullptr) RB_CUDA(cudaMemcpyAsync(&key, device, sizeof key, cudaMemcpyDeviceToHost, s), who);
+    RB_CUDA(cudaStreamSynchronize(s), who);
+    if (mapped != nullptr) key = *static_cast<volatile unsigned int*>(mapped);
+    memcpy(out, &key, sizeof key);
+    return RB_OK;
+  }
+};
+
 bool any_bc(const int32_t* bc, int kind) {
   return bc[0] == kind || bc[1] == kind || bc[2] == kind || bc[3] == kind;
 }
@@ -228,16 +270,14 @@ int rb_li_compute_dt(const rb_li_fields* f, int32_t cur, double alpha, double dt
   if (cur != 0 && cur != 1) return fail(RB_ERR_ARG, "rb_li_compute_dt: cur must be 0 or 1");
   if (!f->h[cur]) return fail(RB_ERR_ARG, "rb_li_compute_dt: missing depth buffer");
   cudaStream_t s = (cudaStream_t)stream;
-  unsigned int* key = &header(ws)->red_key;
   if (f->chan_w && !f->chan_d) return fail(RB_ERR_ARG, "rb_li_compute_dt: chan_w given without chan_d");
   // local_inertial.py:529-539: the water column with channels armed, else h.
-  RB_CUDA(rb::reduce_max_column(f->h[cur], f->chan_w, f->chan_d, (float)f->dx, (size_t)f->ny * f->nx, key, s),
+  const ResultWord word(header(ws));
+  RB_CUDA(rb::reduce_max_column(f->h[cur], f->chan_w, f->chan_d, (float)f->dx, (size_t)f->ny * f->nx,
+                                &header(ws)->max, word.device, s),
           "rb_li_compute_dt reduce");
-  unsigned int host_key = 0;
-  RB_CUDA(cudaMemcpyAsync(&host_key, key, sizeof host_key, cudaMemcpyDeviceToHost, s), "rb_li_compute_dt copy");
-  RB_CUDA(cudaStreamSynchronize(s), "rb_li_compute_dt sync");
   float hmax32;
-  memcpy(&hmax32, &host_key, sizeof hmax32);
+  if ((rc = word.read(&hmax32, s, "rb_li_compute_dt"))) return rc;
   // local_inertial.py:540-544, in host float64 as the reference computes it.
   const double h_max = (double)hmax32;
   if (h_max <= 1.0e-3) {
@@ -325,14 +365,12 @@ int rb_hllc_compute_dt(const rb_hllc_fields* f, int32_t cur, double alpha, doubl
   if (cur != 0 && cur != 1) return fail(RB_ERR_ARG, "rb_hllc_compute_dt: cur must be 0 or 1");
   if (!f->h[cur] || !f->hu[cur] || !f->hv[cur]) return fail(RB_ERR_ARG, "rb_hllc_compute_dt: missing state buffer");
   cudaStream_t s = (cudaStream_t)stream;
-  unsigned int* key = &header(ws)->red_key;
-  RB_CUDA(rb::reduce_wavespeed(f->h[cur], f->hu[cur], f->hv[cur], (size_t)f->ny * f->nx, key, s),
+  const ResultWord word(header(ws));
+  RB_CUDA(rb::reduce_wavespeed(f->h[cur], f->hu[cur], f->hv[cur], (size_t)f->ny * f->nx, &header(ws)->max, word.device,
+                               s),
           "rb_hllc_compute_dt reduce");
-  unsigned int host_key = 0;
-  RB_CUDA(cudaMemcpyAsync(&host_key, key, sizeof host_key, cudaMemcpyDeviceToHost, s), "rb_hllc_compute_dt copy");
-  RB_CUDA(cudaStreamSynchronize(s), "rb_hllc_compute_dt sync");
   float smax32;
-  memcpy(&smax32, &host_key, sizeof smax32);
+  if ((rc = word.read(&smax32, s, "rb_hllc_compute_dt"))) return rc;
   const double smax = (double)smax32;  // hllc.py:987-990
   if (smax <= 0.0) {
     *dt_out = dt_max;
@@ -399,7 +437,7 @@ int rb_li_clock_start(const rb_li_fields* f, int32_t cur, const rb_clock_config*
   cudaStream_t s = (cudaStream_t)stream;
   if ((rc = clock_start(0, f->ny, f->nx, f->dx, cur, cfg, ws, s))) return rc;
   RB_CUDA(rb::reduce_max_column(f->h[cur], f->chan_w, f->chan_d, (float)f->dx, (size_t)f->ny * f->nx,
-                                &header(ws)->clock.red_key, s),
+                                &header(ws)->max, &header(ws)->clock.red_key, s),
           "rb_li_clock_start");
   return RB_OK;
 }
@@ -415,8 +453,8 @@ int rb_hllc_clock_start(const rb_hllc_fields* f, int32_t cur, const rb_clock_con
   cudaStream_t s = (cudaStream_t)stream;
   rb::hllc_prepare_device();
   if ((rc = clock_start(1, f->ny, f->nx, f->dx, cur, cfg, ws, s))) return rc;
-  RB_CUDA(rb::reduce_wavespeed(f->h[cur], f->hu[cur], f->hv[cur], (size_t)f->ny * f->nx, &header(ws)->clock.red_key,
-                               s),
+  RB_CUDA(rb::reduce_wavespeed(f->h[cur], f->hu[cur], f->hv[cur], (size_t)f->ny * f->nx, &header(ws)->max,
+                               &header(ws)->clock.red_key, s),
           "rb_hllc_clock_start");
   return RB_OK;
 }
@@ -476,7 +514,7 @@ int rb_li_clock_reseed(const rb_li_fields* f, int32_t cur, void* ws, void* strea
   if (cur != 0 && cur != 1) return fail(RB_ERR_ARG, "rb_li_clock_reseed: cur must be 0 or 1");
   if (f->chan_w && !f->chan_d) return fail(RB_ERR_ARG, "rb_li_clock_reseed: chan_w given without chan_d");
   RB_CUDA(rb::reduce_max_column(f->h[cur], f->chan_w, f->chan_d, (float)f->dx, (size_t)f->ny * f->nx,
-                                &header(ws)->clock.red_key, (cudaStream_t)stream),
+                                &header(ws)->max, &header(ws)->clock.red_key, (cudaStream_t)stream),
           "rb_li_clock_reseed");
   return RB_OK;
 }
@@ -487,8 +525,8 @@ int rb_hllc_clock_reseed(const rb_hllc_fields* f, int32_t cur, void* ws, void* s
   int rc = check_grid(f->ny, f->nx, f->dx, "rb_hllc_clock_reseed");
   if (rc) return rc;
   if (cur != 0 && cur != 1) return fail(RB_ERR_ARG, "rb_hllc_clock_reseed: cur must be 0 or 1");
-  RB_CUDA(rb::reduce_wavespeed(f->h[cur], f->hu[cur], f->hv[cur], (size_t)f->ny * f->nx, &header(ws)->clock.red_key,
-                               (cudaStream_t)stream),
+  RB_CUDA(rb::reduce_wavespeed(f->h[cur], f->hu[cur], f->hv[cur], (size_t)f->ny * f->nx, &header(ws)->max,
+                               &header(ws)->clock.red_key, (cudaStream_t)stream),
           "rb_hllc_clock_reseed");
   return RB_OK;
 }
@@ -767,10 +805,13 @@ int rb_ensemble_init(rb_ensemble_layout* L, void* ens, const int32_t* scheme, co
   for (int d = 0; d < L->ndom; d++) {
     if (scheme[d] == 0) {
       const rb_li_fields& f = li[ili++];
-      RB_CUDA(rb::reduce_max_h(f.h[cur[d]], (size_t)f.ny * f.nx, &clocks[d].red_key, s), "ens seed");
+      RB_CUDA(rb::reduce_max_column(f.h[cur[d]], nullptr, nullptr, 0.0f, (size_t)f.ny * f.nx, &header(dom_ws[d])->max,
+                                    &clocks[d].red_key, s),
+              "ens seed");
     } else {
       const rb_hllc_fields& f = hl[ihl++];
-      RB_CUDA(rb::reduce_wavespeed(f.h[cur[d]], f.hu[cur[d]], f.hv[cur[d]], (size_t)f.ny * f.nx, &clocks[d].red_key, s),
+      RB_CUDA(rb::reduce_wavespeed(f.h[cur[d]], f.hu[cur[d]], f.hv[cur[d]], (size_t)f.ny * f.nx,
+                                   &header(dom_ws[d])->max, &clocks[d].red_key, s),
               "ens seed");
     }
   }

@@ -183,11 +183,17 @@ int hllc_kernel_variant_count();
 bool hllc_set_kernel_variant(int v);
 void hllc_prepare_device();
 
+// The accumulator of compute_dt's reduction (max of non-negative floats) and its count of
+// finished blocks: zero between calls.
+struct MaxScratch {
+  unsigned int key, ticket;
+};
+
 // Workspace layout (byte offsets from the workspace base).
 struct WsHeader {
-  unsigned int red_key;  // reduction slot (max of non-negative floats)
+  unsigned int red_key;  // compute_dt's result where no mapped host word is to be had
   unsigned int err;      // device error bits
-  unsigned int pad[2];
+  MaxScratch max;
   double sum;            // f64 reduction result
   double pad2[5];
   DevClock clock;        // the device-resident clock (offset 64)
@@ -203,12 +209,11 @@ size_t ws_li_bytes(int ny, int nx);
 size_t ws_hllc_bytes(int ny, int nx);
 size_t ws_hllc_u1_offset(int ny, int nx);
 
-cudaError_t reduce_max_h(const float* h, size_t n, unsigned int* key, cudaStream_t s);
-// Max of the water column (channels.py:73-83) when w is set, else of h.
+// Max of the water column (channels.py:73-83) when w is set, else of h; of the wave speed.
 cudaError_t reduce_max_column(const float* h, const float* w, const float* d, float dx32, size_t n,
-                              unsigned int* key, cudaStream_t s);
-cudaError_t reduce_wavespeed(const float* h, const float* hu, const float* hv, size_t n, unsigned int* key,
-                             cudaStream_t s);
+                              MaxScratch* scratch, unsigned int* out, cudaStream_t s);
+cudaError_t reduce_wavespeed(const float* h, const float* hu, const float* hv, size_t n, MaxScratch* scratch,
+                             unsigned int* out, cudaStream_t s);
 cudaError_t sum_f64(const float* x, size_t n, double* partials, double* out, cudaStream_t s);
 cudaError_t sum_ledger(const double* ledger, size_t nslots, double* partials, double* out, cudaStream_t s);
 cudaError_t reservoir_withdraw(float* h, int nx, int r0, int c0, int rows, int cols, float scale, double* taken,
