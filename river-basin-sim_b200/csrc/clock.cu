@@ -81,6 +81,7 @@ __device__ __forceinline__ int step_limit(int steps, int budget) {
   return m > 2147483647LL ? 2147483647 : (int)m;
 }
 
+// Plan into `c`, all but the two quotients of the new dt (clock_quotients).
 __device__ void clock_plan(DevClock* c) {
   commit(c);
   c->active = 0;
@@ -132,8 +133,6 @@ __device__ void clock_plan(DevClock* c) {
   c->dt = dt;
   c->t1 = t + dt;
   c->dt32 = (float)dt;
-  c->dxdt32 = (float)(dt / c->dx);  // boundaries.py:329
-  c->wt = 0.5 * dt / c->dx;         // hllc.py:1320
   c->rain32 = (float)rain;
   c->scale32 = scale;
   for (int e = 0; e < 4; e++) {  // hllc.py:1308-1312, once per step at the midpoint
@@ -145,16 +144,44 @@ __device__ void clock_plan(DevClock* c) {
   c->pending = 1;
 }
 
-__global__ void clock_plan_kernel(DevClock* c) {
-  pdl_trigger();
-  pdl_wait();
-  clock_plan(c);
+// One warp plans one clock. The clock is fetched and written back as a whole, coalesced,
+// and planned on a copy in shared memory: read field by field the plan was a chain of four
+// or five L2 round trips (3.6 us a step with its launch). Two lanes then divide side by side.
+constexpr int kClockWords = (int)(sizeof(DevClock) / sizeof(unsigned long long));
+static_assert(sizeof(DevClock) % sizeof(unsigned long long) == 0 && kClockWords <= 64, "two words a lane");
+__device__ __forceinline__ void clock_plan_warp(DevClock* clock, DevClock* s, int lane) {
+  auto* g8 = reinterpret_cast<unsigned long long*>(clock);
+  auto* s8 = reinterpret_cast<unsigned long long*>(s);
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+    if (lane + 32 * i < kClockWords) s8[lane + 32 * i] = g8[lane + 32 * i];
+  __syncwarp();
+  if (lane == 0) clock_plan(s);
+  __syncwarp();
+  if (s->active && lane < 2) {
+    const double q = (lane == 0 ? s->dt : 0.5 * s->dt) / s->dx;
+    if (lane == 0) s->dxdt32 = (float)q;  // boundaries.py:329
+    if (lane == 1) s->wt = q;             // hllc.py:1320
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+    if (lane + 32 * i < kClockWords) g8[lane + 32 * i] = s8[lane + 32 * i];
 }
 
-// One plan per domain of an ensemble (each domain has its own clock).
-__global__ void clock_plan_many_kernel(DevClock* clocks, int n) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d < n) clock_plan(&clocks[d]);
+__global__ void __launch_bounds__(32) clock_plan_kernel(DevClock* c) {
+  __shared__ __align__(8) unsigned char raw[sizeof(DevClock)];
+  pdl_trigger();
+  pdl_wait();
+  clock_plan_warp(c, reinterpret_cast<DevClock*>(raw), threadIdx.x);
+}
+
+// One plan per domain of an ensemble (each domain has its own clock), four to a block.
+constexpr int kPlanWarps = 4;
+__global__ void __launch_bounds__(32 * kPlanWarps) clock_plan_many_kernel(DevClock* clocks, int n) {
+  __shared__ __align__(8) unsigned char raw[kPlanWarps][sizeof(DevClock)];
+  const int w = threadIdx.x >> 5, d = blockIdx.x * kPlanWarps + w;
+  if (d < n) clock_plan_warp(&clocks[d], reinterpret_cast<DevClock*>(raw[w]), threadIdx.x & 31);
 }
 
 __global__ void clock_commit_many_kernel(DevClock* clocks, int n) {
@@ -177,7 +204,7 @@ __global__ void clock_target_many_kernel(DevClock* clocks, int n, const double* 
 }
 
 cudaError_t clock_plan_many_launch(DevClock* clocks, int n, cudaStream_t s) {
-  clock_plan_many_kernel<<<(n + 127) / 128, 128, 0, s>>>(clocks, n);
+  clock_plan_many_kernel<<<(n + kPlanWarps - 1) / kPlanWarps, 32 * kPlanWarps, 0, s>>>(clocks, n);
   return cudaGetLastError();
 }
 
@@ -250,7 +277,7 @@ cudaError_t clock_inflow_launch(DevClock* clk, float* const* hb, cudaStream_t s)
 }
 
 cudaError_t clock_plan_launch(DevClock* clk, cudaStream_t s) {
-  return launch_chain(clock_plan_kernel, dim3(1), dim3(1), 0, s, clk);
+  return launch_chain(clock_plan_kernel, dim3(1), dim3(32), 0, s, clk);
 }
 
 cudaError_t clock_commit_launch(DevClock* clk, cudaStream_t s) {

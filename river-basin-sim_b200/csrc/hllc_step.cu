@@ -413,6 +413,38 @@ __device__ __forceinline__ void any_face_flux(const Rec& L, const Rec& R, int ki
   any_face_flux(sides(L, R), kind, low, e, stage, fh, fl, fr, ft, h_l_out, h_r_out);
 }
 
+// The stage's scalars, from the kernel parameters or the device clock.
+struct HllcStageScalars {
+  int cur, rain_mode;
+  float dt, rain32, scale32;
+  float stage[4];  // fixed_stage surfaces, in RB_EDGE order
+  double wt;
+};
+
+__device__ __forceinline__ bool hllc_scalars(const HllcParams& p, HllcStageScalars& s) {
+  s.cur = p.cur;
+  s.rain_mode = p.rain_mode;
+  s.dt = p.dt32;
+  s.rain32 = p.rain32;
+  s.scale32 = p.scale32;
+  s.wt = p.wt;
+#pragma unroll
+  for (int e = 0; e < 4; e++) s.stage[e] = p.stage[e];
+  if (p.clk != nullptr) {  // device-resident clock: this step's dt and forcing, in one round trip
+    const DevClock c = *p.clk;
+    s.cur = c.cur;
+    s.dt = c.dt32;
+    s.wt = c.wt;
+    s.rain32 = c.rain32;
+    s.scale32 = c.scale32;
+    s.rain_mode = (p.h_comp != nullptr && p.rain_field == nullptr) ? 1 : (s.rain32 != 0.0f ? 2 : 0);
+#pragma unroll
+    for (int e = 0; e < 4; e++) s.stage[e] = c.stage32[e];
+    return c.active != 0;
+  }
+  return true;
+}
+
 template <int TX, int TY>
 struct HllcSmem {
   static constexpr int H = 3;                     // halo
@@ -585,25 +617,13 @@ __device__ __forceinline__ bool hllc_tile(const HllcParams& p, int bx, int by, s
 
   const int ny = p.ny, nx = p.nx;
   const int x0 = bx * TX, y0 = by * TY;
-  int cur = p.cur, rain_mode = p.rain_mode;
-  float dt = p.dt32, rain32 = p.rain32, scale32 = p.scale32;
-  float stage_w = p.stage[RB_EDGE_WEST], stage_e = p.stage[RB_EDGE_EAST];
-  float stage_n = p.stage[RB_EDGE_NORTH], stage_s = p.stage[RB_EDGE_SOUTH];
-  double wt = p.wt;
-  if (p.clk != nullptr) {  // device-resident clock: this step's dt and forcing
-    const DevClock* c = p.clk;
-    if (!c->active) return true;
-    cur = c->cur;
-    dt = c->dt32;
-    wt = c->wt;
-    rain32 = c->rain32;
-    scale32 = c->scale32;
-    rain_mode = (p.h_comp != nullptr && p.rain_field == nullptr) ? 1 : (rain32 != 0.0f ? 2 : 0);
-    stage_w = c->stage32[RB_EDGE_WEST];
-    stage_e = c->stage32[RB_EDGE_EAST];
-    stage_n = c->stage32[RB_EDGE_NORTH];
-    stage_s = c->stage32[RB_EDGE_SOUTH];
-  }
+  HllcStageScalars sc;
+  if (!hllc_scalars(p, sc)) return true;
+  const int cur = sc.cur, rain_mode = sc.rain_mode;
+  const float dt = sc.dt, rain32 = sc.rain32, scale32 = sc.scale32;
+  const float stage_w = sc.stage[RB_EDGE_WEST], stage_e = sc.stage[RB_EDGE_EAST];
+  const float stage_n = sc.stage[RB_EDGE_NORTH], stage_s = sc.stage[RB_EDGE_SOUTH];
+  const double wt = sc.wt;
   // Stage input U_s (U^n for stage 1, U1 for stage 2) and U^n.
   const float* __restrict__ h_s = STAGE == 1 ? p.hb[cur] : p.h1;
   const float* __restrict__ hu_s = STAGE == 1 ? p.hub[cur] : p.hu1;

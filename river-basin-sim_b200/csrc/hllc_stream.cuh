@@ -104,37 +104,6 @@ __device__ __forceinline__ Rec recon_diff(const Quad& c, const Quad& dm, const Q
   return r;
 }
 
-struct HllcStageScalars {
-  int cur, rain_mode;
-  float dt, rain32, scale32;
-  float stage[4];  // fixed_stage surfaces, in RB_EDGE order
-  double wt;
-};
-
-__device__ __forceinline__ bool hllc_scalars(const HllcParams& p, HllcStageScalars& s) {
-  s.cur = p.cur;
-  s.rain_mode = p.rain_mode;
-  s.dt = p.dt32;
-  s.rain32 = p.rain32;
-  s.scale32 = p.scale32;
-  s.wt = p.wt;
-#pragma unroll
-  for (int e = 0; e < 4; e++) s.stage[e] = p.stage[e];
-  if (p.clk != nullptr) {  // device-resident clock: this step's dt and forcing
-    const DevClock* c = p.clk;
-    if (!c->active) return false;
-    s.cur = c->cur;
-    s.dt = c->dt32;
-    s.wt = c->wt;
-    s.rain32 = c->rain32;
-    s.scale32 = c->scale32;
-    s.rain_mode = (p.h_comp != nullptr && p.rain_field == nullptr) ? 1 : (s.rain32 != 0.0f ? 2 : 0);
-#pragma unroll
-    for (int e = 0; e < 4; e++) s.stage[e] = c->stage32[e];
-  }
-  return true;
-}
-
 // Rows [i0, i1) of the strip whose first column (lane 0) is c0. EDGE: the strip or its
 // halo may reach a domain edge (clamped indices, edge faces, banking); the other
 // instantiation is for strips whose every staged cell lies inside. Element offsets are

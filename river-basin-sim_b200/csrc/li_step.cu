@@ -113,6 +113,28 @@ __device__ __forceinline__ float combined_capacity(float q_ch, float q_fp, float
   return qs_fp * (1.0f - frac) + qs_ch * frac;
 }
 
+// The step's scalars, from the kernel parameters or the device clock.
+struct LiStepScalars {
+  int cur, limit;
+  float dt, rain_cont, rain32, scale32, dxdt;
+};
+
+__device__ __forceinline__ bool li_scalars(const LiParams& p, LiStepScalars& s) {
+  s = LiStepScalars{p.cur, p.limit, p.dt32, p.rain_cont, p.rain32, p.scale32, p.dxdt};
+  if (p.clk != nullptr) {  // device-resident clock: this step's dt and forcing, in one round trip
+    const DevClock c = *p.clk;
+    s.cur = c.cur;
+    s.limit = c.limit;
+    s.dt = c.dt32;
+    s.rain32 = c.rain32;
+    s.rain_cont = p.h_comp != nullptr ? 0.0f : s.rain32;
+    s.scale32 = c.scale32;
+    s.dxdt = c.dxdt32;
+    return c.active != 0;
+  }
+  return true;
+}
+
 template <int TX, int TY>
 struct LiGeom {
   static constexpr int RW = TX + 4, RH = TY + 4;  // cells: cols x0-2 .. x0+TX+1, rows y0-2 .. y0+TY+1
@@ -173,19 +195,10 @@ __device__ __forceinline__ void li_tile(const LiParams& p, int bx, int by, size_
 
   const int ny = p.ny, nx = p.nx;
   const int x0 = bx * TX, y0 = by * TY;
-  int cur = p.cur, limit = p.limit;
-  float dt = p.dt32, rain_cont = p.rain_cont, rain32 = p.rain32, scale32 = p.scale32, dxdt = p.dxdt;
-  if (p.clk != nullptr) {  // device-resident clock: this step's dt and forcing
-    const DevClock* c = p.clk;
-    if (!c->active) return;
-    cur = c->cur;
-    limit = c->limit;
-    dt = c->dt32;
-    rain32 = c->rain32;
-    rain_cont = p.h_comp != nullptr ? 0.0f : rain32;
-    scale32 = c->scale32;
-    dxdt = c->dxdt32;
-  }
+  LiStepScalars sc;
+  if (!li_scalars(p, sc)) return;
+  const int cur = sc.cur, limit = sc.limit;
+  const float dt = sc.dt, rain_cont = sc.rain_cont, rain32 = sc.rain32, scale32 = sc.scale32, dxdt = sc.dxdt;
   const float* __restrict__ h_in = p.hb[cur];
   const float* __restrict__ qx_in = p.qxb[cur];
   const float* __restrict__ qy_in = p.qyb[cur];

@@ -103,28 +103,6 @@ __device__ __forceinline__ LiFaceConst li_face_const(float dt, float dx) {
   return c;
 }
 
-// The step's scalars, from the kernel parameters or the device clock.
-struct LiStepScalars {
-  int cur, limit;
-  float dt, rain_cont, rain32, scale32, dxdt;
-};
-
-__device__ __forceinline__ bool li_scalars(const LiParams& p, LiStepScalars& s) {
-  s = LiStepScalars{p.cur, p.limit, p.dt32, p.rain_cont, p.rain32, p.scale32, p.dxdt};
-  if (p.clk != nullptr) {  // device-resident clock: this step's dt and forcing
-    const DevClock* c = p.clk;
-    if (!c->active) return false;
-    s.cur = c->cur;
-    s.limit = c->limit;
-    s.dt = c->dt32;
-    s.rain32 = c->rain32;
-    s.rain_cont = p.h_comp != nullptr ? 0.0f : s.rain32;
-    s.scale32 = c->scale32;
-    s.dxdt = c->dxdt32;
-  }
-  return true;
-}
-
 // Per-cell sources of a step: none beyond a uniform rain added plainly, the compensated
 // uniform rain, or whatever the pointers say (rain field, infiltration).
 enum { kLiSrcNone = 0, kLiSrcComp = 1, kLiSrcAny = 2 };
