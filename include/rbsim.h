@@ -234,8 +234,9 @@ int rb_clock_read(void *ws, void *stream, rb_clock_state *out);
 /* --- ensembles and serving ------------------------------------------------------
  * Many independent domains (local inertial and HLLC mixed) stepped together: each
  * keeps its own fields, workspace and device clock (its own dt, rain and target),
- * and one persistent kernel per scheme walks the (domain, tile) work-list of all of
- * them; a domain whose clock has stopped costs one early return per tile. A
+ * and one kernel per scheme walks the (domain, tile) work-list of all of them (large
+ * domains have launches of their own, or a grouped one); a domain whose clock has
+ * stopped costs one early return per tile. A
  * domain's arithmetic is exactly that of rb_li_step / rb_hllc_step, so its result
  * does not depend on the batch it is in. No reference counterpart: the reference
  * runs one scenario per process (solver/run.py:530). The ensemble workspace
@@ -262,8 +263,14 @@ int rb_ensemble_init(rb_ensemble_layout *L, void *ens, const int32_t *scheme, co
 /* Per-domain span targets (host arrays). Synchronising. */
 int rb_ensemble_set_targets(const rb_ensemble_layout *L, void *ens, const double *t_target, const int32_t *max_steps,
                             void *stream);
-/* nsteps x (plan every clock, LI tiles, HLLC stage 1 tiles, HLLC stage 2 tiles). Capturable. */
+/* nsteps x (plan every clock, LI, HLLC stage 1, HLLC stage 2). Capturable. A scheme's
+ * larger domains are stepped by one grouped launch while enough of them are short of
+ * their targets (as of the last rb_ensemble_set_targets or rb_ensemble_read). */
 int rb_ensemble_enqueue(const rb_ensemble_layout *L, void *ens, int32_t nsteps, void *stream);
+/* Which schemes rb_ensemble_enqueue would group now: bit 0 LI, bit 1 HLLC (or a negative
+ * RB_ERR_*). Every grouping computes the same bits: a graph captured under another one
+ * stays right, and is only slower. */
+int rb_ensemble_route(const void *ens);
 /* Commit and read every domain's clock into out[ndom]. Synchronising. */
 int rb_ensemble_read(const rb_ensemble_layout *L, void *ens, rb_clock_state *out, void *stream);
 

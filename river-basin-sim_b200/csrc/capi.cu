@@ -146,6 +146,99 @@ using rb::check_bc;
 using rb::check_dt;
 using rb::check_grid;
 
+static int64_t tiles_of(int ny, int nx, int tx, int ty) {
+  return (int64_t)((nx + tx - 1) / tx) * (int64_t)((ny + ty - 1) / ty);
+}
+
+// A domain of at least this many 32 x 32 tiles fills the GPU by itself: it is stepped
+// by the single-domain kernels, launched for it alone inside the ensemble's step,
+// instead of by the persistent (domain, tile) kernel. Measured on B200 (exact build,
+// Gcell-updates/s, persistent vs single-domain kernel): LI 2048^2 27.6 vs 35.4, 1024^2
+// 27.1 vs 30.0, 512^2 25.5 vs 14.1; HLLC 2048^2 9.9 vs 13.7, 1024^2 9.6 vs 12.1, 512^2
+// 9.2 vs 8.0.
+constexpr int64_t kEnsSoloTiles = 1024;
+
+// How an ensemble's step is launched. A scheme's larger domains (`rows`) can be stepped
+// together by one launch of its row-streaming kernel; otherwise each of kEnsSoloTiles tiles
+// or more has its own launch and the others are on the work-list. The own launches and the
+// work-list hold the domains that are never in `rows` first.
+template <class Params>
+struct EnsRoute {
+  std::vector<Params> rows, own;
+  std::vector<int> row_dom;         // the domains of `rows`
+  int64_t own_rest = 0, tiles_rest = 0, tiles = 0;
+  long long cells_min = 0;
+  bool grouped = false;             // launch `rows` together
+};
+
+// Which domains are grouped, and when: the streaming kernel steps a large amount of work
+// fastest (its rule for one domain), but a domain's step takes a warp's walk down a chunk
+// however small the domain, so that it pays only while the domains still running hold
+// `cells`, and for domains of at least `tiles`; smaller ones join when they are at most a
+// tenth of it, which saves their own launch. Measured on B200 (us per step of n domains of
+// side x side, work-list or own launches / grouped): LI 16 x 256 38.1 / 39.2, 64 x 256
+// 132 / 150, 25 x 400 130 / 120, 4 x 512 37.3 / 35.4, 10 x 600 112 / 87, 6 x 860 133 / 113,
+// 4 x 1000 119 / 98; HLLC 64 x 256 366 / 535, 25 x 400 362 / 417, 3 x 1000 248 / 241,
+// 10 x 600 316 / 292, 6 x 860 378 / 333, 4 x 1000 331 / 306. One domain left of a group:
+// LI 400 15.5 / 33, HLLC 400 33 / 81.
+struct EnsRowRule {
+  int64_t tiles;
+  long long cells;
+};
+constexpr EnsRowRule kEnsLiRows{160, 1500000}, kEnsHllcRows{324, 3000000};
+static bool ens_rows_fit(const rb::LiParams& p) { return rb::ens_li_stream_fits(p); }
+static bool ens_rows_fit(const rb::HllcParams& p) { return rb::ens_hllc_stream_fits(p); }
+
+// `domains[i]` is the ensemble's domain dom[i]; its (i, tile) items go to `map`.
+template <class Params>
+static EnsRoute<Params> ens_route(const std::vector<Params>& domains, const std::vector<int>& dom, EnsRowRule rule,
+                                  int tx, int ty, std::vector<int2>& map) {
+  EnsRoute<Params> r;
+  r.cells_min = rule.cells;
+  const size_t n = domains.size();
+  std::vector<char> grouped(n, 0);
+  long long large = 0, small = 0;
+  for (size_t i = 0; i < n; i++) {
+    const Params& p = domains[i];
+    if (!ens_rows_fit(p)) continue;
+    (tiles_of(p.ny, p.nx, 32, 32) >= rule.tiles ? large : small) += (long long)p.ny * p.nx;
+  }
+  for (size_t i = 0; i < n && large >= rule.cells; i++) {
+    const Params& p = domains[i];
+    grouped[i] = ens_rows_fit(p) && (tiles_of(p.ny, p.nx, 32, 32) >= rule.tiles || 10 * small <= large);
+    if (!grouped[i]) continue;
+    r.rows.push_back(p);
+    r.row_dom.push_back(dom[i]);
+  }
+  r.grouped = !r.rows.empty();
+  for (int pass = 0; pass < 2; pass++) {
+    for (size_t i = 0; i < n; i++) {
+      const Params& p = domains[i];
+      if (grouped[i] != pass) continue;
+      if (tiles_of(p.ny, p.nx, 32, 32) >= kEnsSoloTiles) {
+        r.own.push_back(p);
+      } else {
+        const int64_t nt = tiles_of(p.ny, p.nx, tx, ty);
+        for (int64_t t = 0; t < nt; t++) map.push_back(make_int2((int)i, (int)t));
+      }
+    }
+    if (pass == 0) r.own_rest = (int64_t)r.own.size(), r.tiles_rest = (int64_t)map.size();
+  }
+  r.tiles = (int64_t)map.size();
+  return r;
+}
+
+// Group a scheme's domains while those still short of their targets are enough.
+template <class Params>
+static void ens_regroup(EnsRoute<Params>& r, const std::vector<rb::DevClock>& clocks) {
+  long long cells = 0;
+  for (size_t i = 0; i < r.rows.size(); i++) {
+    const rb::DevClock& c = clocks[r.row_dom[i]];
+    if (c.t < c.t_target && c.steps < c.max_steps) cells += (long long)r.rows[i].ny * r.rows[i].nx;
+  }
+  r.grouped = !r.rows.empty() && cells >= r.cells_min;
+}
+
 extern "C" {
 
 int rb_last_error(char* buf, size_t n) {
@@ -616,23 +709,11 @@ int rb_clock_read(void* ws, void* stream, rb_clock_state* out) {
 }
 
 // --- ensembles ----------------------------------------------------------------
-static int64_t tiles_of(int ny, int nx, int tx, int ty) {
-  return (int64_t)((nx + tx - 1) / tx) * (int64_t)((ny + ty - 1) / ty);
-}
-
-// A domain of at least this many 32 x 32 tiles fills the GPU by itself: it is stepped
-// by the single-domain kernels, launched for it alone inside the ensemble's step,
-// instead of by the persistent (domain, tile) kernel. Measured on B200 (exact build,
-// Gcell-updates/s, persistent vs single-domain kernel): LI 2048^2 27.6 vs 35.4, 1024^2
-// 27.1 vs 30.0, 512^2 25.5 vs 14.1; HLLC 2048^2 9.9 vs 13.7, 1024^2 9.6 vs 12.1, 512^2
-// 9.2 vs 8.0.
-constexpr int64_t kEnsSoloTiles = 1024;
-
-// The single-domain launch parameters of an ensemble's large domains, by ensemble
-// buffer (kernel parameters are passed by value, so the host keeps them).
+// The launches of an ensemble's step, by ensemble buffer (kernel parameters are passed by
+// value, so the host keeps them).
 struct EnsSolo {
-  std::vector<rb::LiParams> li;
-  std::vector<rb::HllcParams> hllc;
+  EnsRoute<rb::LiParams> li;
+  EnsRoute<rb::HllcParams> hllc;
 };
 static std::mutex g_ens_solo_mu;
 static std::unordered_map<const void*, EnsSolo> g_ens_solo;
@@ -706,13 +787,6 @@ int rb_ensemble_init(rb_ensemble_layout* L, void* ens, const int32_t* scheme, co
   std::vector<rb::DevClock> hc(L->ndom);
   std::vector<rb::LiParams> hli(L->n_li);
   std::vector<rb::HllcParams> hhl(L->n_hllc);
-  std::vector<int2> mli, mhl;
-  mli.reserve((size_t)L->li_tiles);
-  mhl.reserve((size_t)L->hllc_tiles);
-  int ltx, lty, htx, hty;
-  rb::li_variant_tile(L->li_variant, &ltx, &lty);
-  rb::hllc_variant_tile(L->hllc_variant, &htx, &hty);
-  EnsSolo solo;
   int ili = 0, ihl = 0;
   for (int d = 0; d < L->ndom; d++) {
     if (!dom_ws[d]) return fail(RB_ERR_ARG, "rb_ensemble_init: domain %d has no workspace", d);
@@ -730,12 +804,6 @@ int rb_ensemble_init(rb_ensemble_layout* L, void* ens, const int32_t* scheme, co
       hli[ili].clk = &clocks[d];
       hli[ili].hmax_key = &clocks[d].red_key;
       ny = f.ny, nx = f.nx, dx = f.dx;
-      if (tiles_of(ny, nx, 32, 32) >= kEnsSoloTiles) {
-        solo.li.push_back(hli[ili]);
-      } else {
-        const int64_t nt = tiles_of(ny, nx, ltx, lty);
-        for (int64_t t = 0; t < nt; t++) mli.push_back(make_int2(ili, (int)t));
-      }
       ili++;
     } else {
       const rb_hllc_fields& f = hl[ihl];
@@ -743,12 +811,6 @@ int rb_ensemble_init(rb_ensemble_layout* L, void* ens, const int32_t* scheme, co
       hhl[ihl].clk = &clocks[d];
       hhl[ihl].smax_key = &clocks[d].red_key;
       ny = f.ny, nx = f.nx, dx = f.dx;
-      if (tiles_of(ny, nx, 32, 32) >= kEnsSoloTiles) {
-        solo.hllc.push_back(hhl[ihl]);
-      } else {
-        const int64_t nt = tiles_of(ny, nx, htx, hty);
-        for (int64_t t = 0; t < nt; t++) mhl.push_back(make_int2(ihl, (int)t));
-      }
       ihl++;
     }
     if (!(k.alpha > 0.0) || !(k.dt_max > 0.0)) return fail(RB_ERR_ARG, "rb_ensemble_init: domain %d alpha/dt_max", d);
@@ -772,6 +834,17 @@ int rb_ensemble_init(rb_ensemble_layout* L, void* ens, const int32_t* scheme, co
     c.limit = k.limit ? 1 : 0;
     hc[d] = c;
   }
+  std::vector<int2> mli, mhl;
+  mli.reserve((size_t)L->li_tiles);
+  mhl.reserve((size_t)L->hllc_tiles);
+  int ltx, lty, htx, hty;
+  rb::li_variant_tile(L->li_variant, &ltx, &lty);
+  rb::hllc_variant_tile(L->hllc_variant, &htx, &hty);
+  std::vector<int> dom_li, dom_hllc;
+  for (int d = 0; d < L->ndom; d++) (scheme[d] == 0 ? dom_li : dom_hllc).push_back(d);
+  EnsSolo solo;
+  solo.li = ens_route(hli, dom_li, kEnsLiRows, ltx, lty, mli);
+  solo.hllc = ens_route(hhl, dom_hllc, kEnsHllcRows, htx, hty, mhl);
   if ((int64_t)mli.size() > L->li_tiles || (int64_t)mhl.size() > L->hllc_tiles)
     return fail(RB_ERR_ARG, "rb_ensemble_init: the domains have more tiles than the layout was made for");
   // the persistent kernels walk the small domains' tiles only
@@ -830,6 +903,14 @@ int rb_ensemble_set_targets(const rb_ensemble_layout* L, void* ens, const double
   RB_CUDA(cudaMemcpyAsync(dm, max_steps, (size_t)L->ndom * sizeof(int32_t), cudaMemcpyHostToDevice, s), "targets");
   RB_CUDA(rb::clock_target_many_launch((rb::DevClock*)(base + L->off_clocks), L->ndom, dt_t, dm, s), "targets");
   RB_CUDA(cudaStreamSynchronize(s), "rb_ensemble_set_targets sync");
+  {
+    std::lock_guard<std::mutex> lock(g_ens_solo_mu);
+    auto it = g_ens_solo.find(ens);
+    if (it != g_ens_solo.end()) {
+      it->second.li.grouped = !it->second.li.rows.empty();
+      it->second.hllc.grouped = !it->second.hllc.rows.empty();
+    }
+  }
   return RB_OK;
 }
 
@@ -850,18 +931,31 @@ int rb_ensemble_enqueue(const rb_ensemble_layout* L, void* ens, int32_t nsteps, 
     solo = it->second;
   }
   const int li_v = rb::li_current_variant(), hl_v = rb::hllc_current_variant();
+  const auto& li = solo.li;
+  const auto& hl = solo.hllc;
+  const int n_li = li.grouped ? (int)li.rows.size() : 0, n_hl = hl.grouped ? (int)hl.rows.size() : 0;
+  const size_t own_li = li.grouped ? li.own_rest : li.own.size(), own_hl = hl.grouped ? hl.own_rest : hl.own.size();
+  const int64_t tiles_li = li.grouped ? li.tiles_rest : li.tiles, tiles_hl = hl.grouped ? hl.tiles_rest : hl.tiles;
   for (int k = 0; k < nsteps; k++) {
     RB_CUDA(rb::clock_plan_many_launch(clocks, L->ndom, s), "ens plan");
-    for (const rb::LiParams& p : solo.li) RB_CUDA(rb::li_step_launch_variant(p, li_v, s), "ens li, large domain");
-    RB_CUDA(rb::ens_li_launch(L->li_variant, L->li_grid, P, mli, L->li_tiles, s), "ens li");
-    for (const rb::HllcParams& p : solo.hllc)
-      RB_CUDA(rb::hllc_stage_launch_exact(p, 1, hl_v, s), "ens hllc 1, large domain");
-    RB_CUDA(rb::ens_hllc_launch(L->hllc_variant, L->hllc_grid, 1, Q, mhl, L->hllc_tiles, s), "ens hllc 1");
-    for (const rb::HllcParams& p : solo.hllc)
-      RB_CUDA(rb::hllc_stage_launch_exact(p, 2, hl_v, s), "ens hllc 2, large domain");
-    RB_CUDA(rb::ens_hllc_launch(L->hllc_variant, L->hllc_grid, 2, Q, mhl, L->hllc_tiles, s), "ens hllc 2");
+    RB_CUDA(rb::ens_li_stream_launch(li.rows.data(), n_li, s), "ens li, grouped domains");
+    for (size_t i = 0; i < own_li; i++) RB_CUDA(rb::li_step_launch_variant(li.own[i], li_v, s), "ens li, large domain");
+    RB_CUDA(rb::ens_li_launch(L->li_variant, L->li_grid, P, mli, tiles_li, s), "ens li");
+    for (int stage = 1; stage <= 2; stage++) {
+      RB_CUDA(rb::ens_hllc_stream_launch(hl.rows.data(), n_hl, stage, s), "ens hllc, grouped domains");
+      for (size_t i = 0; i < own_hl; i++)
+        RB_CUDA(rb::hllc_stage_launch_exact(hl.own[i], stage, hl_v, s), "ens hllc, large domain");
+      RB_CUDA(rb::ens_hllc_launch(L->hllc_variant, L->hllc_grid, stage, Q, mhl, tiles_hl, s), "ens hllc");
+    }
   }
   return RB_OK;
+}
+
+int rb_ensemble_route(const void* ens) {
+  std::lock_guard<std::mutex> lock(g_ens_solo_mu);
+  auto it = g_ens_solo.find(ens);
+  if (it == g_ens_solo.end()) return fail(RB_ERR_ARG, "rb_ensemble_route: the ensemble was not initialised");
+  return (it->second.li.grouped ? 1 : 0) | (it->second.hllc.grouped ? 2 : 0);
 }
 
 int rb_ensemble_read(const rb_ensemble_layout* L, void* ens, rb_clock_state* out, void* stream) {
@@ -872,6 +966,14 @@ int rb_ensemble_read(const rb_ensemble_layout* L, void* ens, rb_clock_state* out
   std::vector<rb::DevClock> hc(L->ndom);
   RB_CUDA(cudaMemcpyAsync(hc.data(), clocks, hc.size() * sizeof(rb::DevClock), cudaMemcpyDeviceToHost, s), "ens read");
   RB_CUDA(cudaStreamSynchronize(s), "rb_ensemble_read sync");
+  {
+    std::lock_guard<std::mutex> lock(g_ens_solo_mu);
+    auto it = g_ens_solo.find(ens);
+    if (it != g_ens_solo.end()) {
+      ens_regroup(it->second.li, hc);
+      ens_regroup(it->second.hllc, hc);
+    }
+  }
   for (int d = 0; d < L->ndom; d++) {
     out[d].t = hc[d].t;
     out[d].dt = hc[d].dt;

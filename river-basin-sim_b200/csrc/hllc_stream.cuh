@@ -366,20 +366,15 @@ __device__ __forceinline__ void hllc_stream_strip(const HllcParams& p, const Hll
   if (!EDGE && !own) smax = 0.0f, bad = false;
 }
 
-// One warp a block (no sibling to wait for at the end), 16 resident per SM: at 20 and 24
-// (96 and 80 registers) the schedulers have no more to issue and the spills show (2048^2
-// dam break, us per step, fast / exact: 189.7 / 270 for 16, 198.8 / 296 for 20, 209.9 / 308
-// for 24).
-constexpr int kHllcStreamWarps = 16;
+// One block's strip and chunk. `order` counts chunks as they are started: the last one
+// runs second, since the domain's top and bottom chunks are the slow ones.
 template <int STAGE, int SRC>
-__global__ void __launch_bounds__(32, kHllcStreamWarps) hllc_stream_kernel(const HllcParams p, int rows) {
-  __shared__ HllcRing<STAGE, SRC> ring;
-  pdl_wait();
+__device__ __forceinline__ void hllc_stream_block(const HllcParams& p, int strip, int order, int chunks, size_t slot,
+                                                  int rows, HllcRing<STAGE, SRC>& ring) {
   HllcStageScalars s;
   if (!hllc_scalars(p, s)) return;
-  const int c0 = blockIdx.x * kHllcStreamCols - kHllcHalo;
-  // the last chunk runs second: the domain's top and bottom chunks are the slow ones
-  const int chunk = blockIdx.y == 1 ? gridDim.y - 1 : (blockIdx.y > 1 ? blockIdx.y - 1 : 0);
+  const int c0 = strip * kHllcStreamCols - kHllcHalo;
+  const int chunk = order == 1 ? chunks - 1 : (order > 1 ? order - 1 : 0);
   const int i0 = chunk * rows, i1 = min(p.ny, i0 + rows);
   double loss = 0.0;
   float smax = 0.0f;
@@ -393,7 +388,7 @@ __global__ void __launch_bounds__(32, kHllcStreamWarps) hllc_stream_kernel(const
   const int lane = threadIdx.x;
   if (p.ledger != nullptr) {
     const double t = warp_sum(loss);
-    if (lane == 0) ledger_add(p.ledger + 2 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x), t);
+    if (lane == 0) ledger_add(p.ledger + 2 * slot, t);
   }
   if (STAGE == 2) {
     if (p.smax_key != nullptr) {
@@ -402,6 +397,19 @@ __global__ void __launch_bounds__(32, kHllcStreamWarps) hllc_stream_kernel(const
     }
     if (bad) flag_error(p.err, RB_DEVERR_NONFINITE);
   }
+}
+
+// One warp a block (no sibling to wait for at the end), 16 resident per SM: at 20 and 24
+// (96 and 80 registers) the schedulers have no more to issue and the spills show (2048^2
+// dam break, us per step, fast / exact: 189.7 / 270 for 16, 198.8 / 296 for 20, 209.9 / 308
+// for 24).
+constexpr int kHllcStreamWarps = 16;
+template <int STAGE, int SRC>
+__global__ void __launch_bounds__(32, kHllcStreamWarps) hllc_stream_kernel(const HllcParams p, int rows) {
+  __shared__ HllcRing<STAGE, SRC> ring;
+  pdl_wait();
+  hllc_stream_block<STAGE, SRC>(p, blockIdx.x, blockIdx.y, gridDim.y, (size_t)blockIdx.y * gridDim.x + blockIdx.x,
+                                rows, ring);
 }
 
 static cudaError_t launch_hllc_stream(const HllcParams& p, int stage, cudaStream_t s) {
@@ -427,3 +435,57 @@ constexpr long long kHllcStreamCells = 3000000;
 static bool hllc_stream_takes(const HllcParams& p) {
   return (long long)p.ny * p.nx >= kHllcStreamCells && p.nx >= 30 * kHllcStreamCols && hllc_stream_fits(p.ny, p.nx);
 }
+
+#if !defined(RB_FAST_MATH)
+// The larger domains of an ensemble in one launch: together they fill the GPU where each
+// alone would leave part of its last wave, or all of it, idle (a mix of 20 domains of 128^2
+// to 1364^2, us per step: 545 with a launch for each of the three largest and a work-list of
+// tiles for the rest, 460 with a launch per scheme and stage).
+template <int STAGE, int SRC>
+__global__ void __launch_bounds__(32, kHllcStreamWarps)
+    ens_hllc_stream_kernel(const __grid_constant__ StreamGroup<HllcParams> g) {
+  __shared__ HllcRing<STAGE, SRC> ring;
+  pdl_wait();
+  int d = 0;
+  while ((int)blockIdx.x >= g.first[d + 1]) d++;
+  const HllcParams& p = g.p[d];
+  const int strips = (p.nx + kHllcStreamCols - 1) / kHllcStreamCols;
+  const int b = blockIdx.x - g.first[d];
+  hllc_stream_block<STAGE, SRC>(p, b % strips, b / strips, (p.ny + g.rows - 1) / g.rows, (size_t)b, g.rows, ring);
+}
+
+constexpr int kEnsHllcMinRows = 11;  // 26 x 11 cells a block: what the ledger's slots allow
+bool ens_hllc_stream_fits(const HllcParams& p) {
+  const long long blocks = (long long)((p.nx + kHllcStreamCols - 1) / kHllcStreamCols) *
+                           ((p.ny + kEnsHllcMinRows - 1) / kEnsHllcMinRows);
+  return blocks <= (long long)((p.nx + 31) / 32) * ((p.ny + 7) / 8) && (48 + 16LL) * p.nx < (1LL << 31) &&
+         blocks < (1LL << 31) / kStreamGroup;
+}
+
+cudaError_t ens_hllc_stream_launch(const HllcParams* p, int n, int stage, cudaStream_t s) {
+  const int groups = (n + kStreamGroup - 1) / kStreamGroup;
+  for (int k = 0; k < groups; k++) {
+    const int d0 = (int)((long long)n * k / groups), m = (int)((long long)n * (k + 1) / groups) - d0;
+    StreamGroup<HllcParams> g{};
+    long long strip_rows = 0;
+    bool src = false;
+    for (int d = 0; d < m; d++) {
+      const HllcParams& q = g.p[d] = p[d0 + d];
+      strip_rows += (long long)((q.nx + kHllcStreamCols - 1) / kHllcStreamCols) * q.ny;
+      src |= q.h_comp != nullptr || q.rain_field != nullptr || q.infil != nullptr;
+    }
+    const long long rows = (strip_rows + 2 * 148 * 16 - 1) / (2 * 148 * 16);
+    g.rows = (int)(rows < kEnsHllcMinRows ? kEnsHllcMinRows : (rows > 48 ? 48 : rows));
+    for (int d = 0; d < kStreamGroup; d++)
+      g.first[d + 1] = g.first[d] + (d < m ? ((g.p[d].nx + kHllcStreamCols - 1) / kHllcStreamCols) *
+                                                 ((g.p[d].ny + g.rows - 1) / g.rows)
+                                           : 0);
+    const dim3 grid(g.first[m]), block(32);
+    const cudaError_t e = stage == 1 ? launch_chain(ens_hllc_stream_kernel<1, 0>, grid, block, 0, s, g)
+                          : src      ? launch_chain(ens_hllc_stream_kernel<2, 1>, grid, block, 0, s, g)
+                                     : launch_chain(ens_hllc_stream_kernel<2, 0>, grid, block, 0, s, g);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+#endif

@@ -350,17 +350,15 @@ __device__ __forceinline__ void li_stream_strip(const LiParams& p, const LiStepS
   }
 }
 
-// One warp a block: a block's warps would wait for its slowest strip before the
-// reductions below (14 % of the warp cycles with four warps a block).
+// One block's strip and chunk. `order` counts chunks as they are started: the last one
+// runs second, since the domain's top and bottom chunks are the slow ones.
 template <int SED, int SRC>
-__global__ void __launch_bounds__(32, kLiStreamWarps) li_stream_kernel(const LiParams p, int rows) {
-  __shared__ LiRing<SED, SRC> ring;
-  pdl_wait();
+__device__ __forceinline__ void li_stream_block(const LiParams& p, int strip, int order, int chunks, size_t slot,
+                                                int rows, LiRing<SED, SRC>& ring) {
   LiStepScalars s;
   if (!li_scalars(p, s)) return;
-  const int c0 = blockIdx.x * kLiStreamCols - kLiHalo;
-  // the last chunk runs second: the domain's top and bottom chunks are the slow ones
-  const int chunk = blockIdx.y == 1 ? gridDim.y - 1 : (blockIdx.y > 1 ? blockIdx.y - 1 : 0);
+  const int c0 = strip * kLiStreamCols - kLiHalo;
+  const int chunk = order == 1 ? chunks - 1 : (order > 1 ? order - 1 : 0);
   const int i0 = chunk * rows, i1 = min(p.ny, i0 + rows);
   double loss = 0.0;
   float hmax = 0.0f;
@@ -374,13 +372,23 @@ __global__ void __launch_bounds__(32, kLiStreamWarps) li_stream_kernel(const LiP
   const int lane = threadIdx.x;
   if (p.ledger != nullptr) {
     const double t = warp_sum(loss);
-    if (lane == 0) ledger_add(p.ledger + 2 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x), t);
+    if (lane == 0) ledger_add(p.ledger + 2 * slot, t);
   }
   if (p.hmax_key != nullptr) {
     hmax = warp_max(hmax);
     if (lane == 0) atomicMax(p.hmax_key, max_key(hmax));
   }
   if (bad) flag_error(p.err, RB_DEVERR_NONFINITE);
+}
+
+// One warp a block: a block's warps would wait for its slowest strip before the
+// reductions above (14 % of the warp cycles with four warps a block).
+template <int SED, int SRC>
+__global__ void __launch_bounds__(32, kLiStreamWarps) li_stream_kernel(const LiParams p, int rows) {
+  __shared__ LiRing<SED, SRC> ring;
+  pdl_wait();
+  li_stream_block<SED, SRC>(p, blockIdx.x, blockIdx.y, gridDim.y, (size_t)blockIdx.y * gridDim.x + blockIdx.x, rows,
+                            ring);
 }
 
 // Rows a warp walks: as many warps as the GPU holds at once, within 8 .. 48 (four rows
@@ -422,3 +430,58 @@ static cudaError_t launch_li_stream(const LiParams& p, cudaStream_t s) {
   if (p.h_comp != nullptr) return launch_chain(li_stream_kernel<0, kLiSrcComp>, grid, block, 0, s, p, rows);
   return launch_chain(li_stream_kernel<0, kLiSrcNone>, grid, block, 0, s, p, rows);
 }
+
+#if !defined(RB_FAST_MATH)
+// The larger domains of an ensemble in one launch: together they fill the GPU where each
+// alone would leave part of its last wave, or all of it, idle (a mix of 20 domains of 128^2
+// to 1364^2, us per step: 545 with a launch for each of the three largest and a work-list of
+// tiles for the rest, 460 with a launch per scheme and stage).
+template <int SRC>
+__global__ void __launch_bounds__(32, kLiStreamWarps)
+    ens_li_stream_kernel(const __grid_constant__ StreamGroup<LiParams> g) {
+  __shared__ LiRing<0, SRC> ring;
+  pdl_wait();
+  int d = 0;
+  while ((int)blockIdx.x >= g.first[d + 1]) d++;
+  const LiParams& p = g.p[d];
+  const int strips = (p.nx + kLiStreamCols - 1) / kLiStreamCols;
+  const int b = blockIdx.x - g.first[d];
+  li_stream_block<0, SRC>(p, b % strips, b / strips, (p.ny + g.rows - 1) / g.rows, (size_t)b, g.rows, ring);
+}
+
+constexpr int kEnsLiMinRows = 12;  // 28 x 12 cells a block: what the ledger's slots allow
+bool ens_li_stream_fits(const LiParams& p) {
+  const long long blocks = (long long)((p.nx + kLiStreamCols - 1) / kLiStreamCols) *
+                           ((p.ny + kEnsLiMinRows - 1) / kEnsLiMinRows);
+  return p.d50 == nullptr && p.cw == nullptr && blocks <= (long long)((p.nx + 31) / 32) * ((p.ny + 7) / 8) &&
+         (48 + 8LL) * (p.nx + 1) < (1LL << 31) && blocks < (1LL << 31) / kStreamGroup;
+}
+
+cudaError_t ens_li_stream_launch(const LiParams* p, int n, cudaStream_t s) {
+  const int groups = (n + kStreamGroup - 1) / kStreamGroup;
+  for (int k = 0; k < groups; k++) {
+    const int d0 = (int)((long long)n * k / groups), m = (int)((long long)n * (k + 1) / groups) - d0;
+    StreamGroup<LiParams> g{};
+    long long strip_rows = 0;
+    bool any = false, comp = true;
+    for (int d = 0; d < m; d++) {
+      const LiParams& q = g.p[d] = p[d0 + d];
+      strip_rows += (long long)((q.nx + kLiStreamCols - 1) / kLiStreamCols) * q.ny;
+      any |= q.rain_field != nullptr || q.infil != nullptr || (q.h_comp != nullptr) != (g.p[0].h_comp != nullptr);
+      comp = comp && q.h_comp != nullptr;
+    }
+    const long long rows = (strip_rows + 148LL * kLiStreamWarps - 1) / (148LL * kLiStreamWarps);
+    g.rows = (int)(rows < kEnsLiMinRows ? kEnsLiMinRows : (rows > 48 ? 48 : rows));
+    for (int d = 0; d < kStreamGroup; d++)
+      g.first[d + 1] = g.first[d] + (d < m ? ((g.p[d].nx + kLiStreamCols - 1) / kLiStreamCols) *
+                                                 ((g.p[d].ny + g.rows - 1) / g.rows)
+                                           : 0);
+    const dim3 grid(g.first[m]), block(32);
+    const cudaError_t e = any    ? launch_chain(ens_li_stream_kernel<kLiSrcAny>, grid, block, 0, s, g)
+                          : comp ? launch_chain(ens_li_stream_kernel<kLiSrcComp>, grid, block, 0, s, g)
+                                 : launch_chain(ens_li_stream_kernel<kLiSrcNone>, grid, block, 0, s, g);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+#endif

@@ -119,6 +119,19 @@ inline bool hllc_stream_fits(int ny, int nx) {
          (long long)(rows + 16) * nx < (1LL << 31);
 }
 
+// Domains of an ensemble that one launch of a row-streaming kernel steps together: their
+// parameters by value, as in a domain's own launch, domain d's strips and chunks being
+// blocks first[d] .. first[d + 1].
+constexpr int kStreamGroup = 32;
+template <class Params>
+struct StreamGroup {
+  Params p[kStreamGroup];
+  int first[kStreamGroup + 1];
+  int rows;
+};
+static_assert(sizeof(StreamGroup<LiParams>) <= 32764 && sizeof(StreamGroup<HllcParams>) <= 32764,
+              "what a launch may pass by value");
+
 // The tile of the default HLLC variant below the streaming kernel's sizes: 0 = 16 x 16
 // (704 threads, one pass over its 684 faces), 1 = 32 x 16, 2 = 32 x 32 (640 threads). Few
 // large tiles leave most SMs idle and a stage is one tile's latency (dam break, us per
@@ -169,6 +182,12 @@ void set_last_error(const char* msg);  // the message rb_last_error returns on t
 int check_grid(int ny, int nx, double dx, const char* who);
 int check_bc(const int32_t* bc, bool allow_stage, const char* who);
 int check_dt(double dt, const char* who);
+// Whether an ensemble's domain can be stepped by a grouped launch of the streaming kernel
+// (exact build), and that launch for any number of domains.
+bool ens_li_stream_fits(const LiParams& p);
+bool ens_hllc_stream_fits(const HllcParams& p);
+cudaError_t ens_li_stream_launch(const LiParams* p, int n, cudaStream_t s);
+cudaError_t ens_hllc_stream_launch(const HllcParams* p, int n, int stage, cudaStream_t s);
 int hllc_tiles(int ny, int nx);
 // The HLLC stage-kernel variant in force now; the launch and tile count of one call
 // can take it once, so a concurrent rb_hllc_set_kernel_variant cannot split them.

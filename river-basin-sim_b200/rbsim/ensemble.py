@@ -2,13 +2,14 @@
 
 Each member is an ordinary ``State`` (local inertial or HLLC) with its own
 workspace, rain and horizon; the ensemble gives every member its own device clock
-and steps all of them with one persistent kernel per scheme over a (domain, tile)
-work-list (librbsim ``rb_ensemble_*``), ``graph_steps`` ensemble steps per CUDA
-graph replay. A member of 1024 tiles of 32 x 32 or more fills the GPU by itself and
-is stepped by the single-domain kernels, launched for it alone in the same step
-(faster than the persistent kernels at that size on B200). A member's arithmetic is that of its single-domain step, so its
-result is bit-identical to running it alone; members that reach their target stop
-(their tiles return immediately) while the others continue.
+and steps all of them (librbsim ``rb_ensemble_*``), ``graph_steps`` ensemble steps per CUDA graph
+replay. The larger members of a scheme are stepped together by one launch of its
+row-streaming kernel while enough of them are short of their targets; otherwise a
+member of 1024 tiles of 32 x 32 or more is stepped by the single-domain kernels,
+launched for it alone, and the rest by one kernel per scheme over a (domain, tile)
+work-list. A member's arithmetic is that of its single-domain step, so its result is
+bit-identical to running it alone; members that reach their target stop (their blocks
+return immediately) while the others continue.
 
 ``autotune`` picks the tile shapes of the two persistent kernels by timing each
 candidate on the run itself (tile shape changes which CTA computes a cell, never
@@ -80,7 +81,7 @@ class Ensemble:
         stream = torch.cuda.current_stream(dev).cuda_stream
         _lib.check(self._L.rb_ensemble_init(ctypes.byref(self.layout), self._ws.data_ptr(), self._scheme, self._li,
                                             self._hl, self._wss, cfgs, cur, stream))  # fmt: skip
-        self._graph = None
+        self._graphs = {}  # by how the library would launch a step now
         self.clock = (_lib.ClockState * n)()
 
     def _stream(self) -> int:
@@ -95,12 +96,15 @@ class Ensemble:
                                                    self._stream()))  # fmt: skip
 
     def replay(self) -> None:
-        if self._graph is None:
-            self._graph = graphs.capture(
+        route = self._L.rb_ensemble_route(self._ws.data_ptr())
+        if route < 0:
+            _lib.check(route)
+        if route not in self._graphs:
+            self._graphs[route] = graphs.capture(
                 self.device,
                 lambda s: _lib.check(self._L.rb_ensemble_enqueue(ctypes.byref(self.layout), self._ws.data_ptr(),
                                                                  self.graph_steps, s)))  # fmt: skip
-        self._graph.replay()
+        self._graphs[route].replay()
 
     def read(self):
         _lib.check(self._L.rb_ensemble_read(ctypes.byref(self.layout), self._ws.data_ptr(), self.clock,
