@@ -36,6 +36,7 @@
 namespace rb {
 RB_ARITH_BEGIN
 
+#include "pair.cuh"
 #include "warp_stream.cuh"
 
 // hllc.py:158-165 _minmod
@@ -199,6 +200,40 @@ __device__ __forceinline__ void hllc_near(float hl, float ul, float vtl, float h
   f2 = none ? 0.0f : fh * (star_nonneg ? vtl : vtr);
 }
 
+// hllc_near for the two faces that are the halves of its operands (to rounding).
+__device__ __forceinline__ void hllc_near2(F2 hl, F2 ul, F2 vtl, F2 hr, F2 ur, F2 vtr, F2& f0, F2& f1, F2& f2, bool&) {
+  const float g = kG;
+  const F2 gl = g * F2{fmaxf(hl.x, 0.0f), fmaxf(hl.y, 0.0f)}, gr = g * F2{fmaxf(hr.x, 0.0f), fmaxf(hr.y, 0.0f)};
+  const F2 cl{sqrt_near(gl.x), sqrt_near(gl.y)}, cr{sqrt_near(gr.x), sqrt_near(gr.y)};
+  const bool dlx = hl.x <= kHDry, dly = hl.y <= kHDry, drx = hr.x <= kHDry, dry = hr.y <= kHDry;
+  const F2 hs = fma2(both(0.25f), ul - ur, 0.5f * (cl + cr)), usum = ul + ur;
+  const F2 c_star{fabsf(hs.x), fabsf(hs.y)}, u_star = fma2(both(0.5f), usum, cl - cr);
+  const F2 ulm = ul - cl, urp = ur + cr, sm = u_star - c_star, sp = u_star + c_star;
+  const F2 ul2 = fma2(both(2.0f), cl, ul), ur2 = fma2(both(-2.0f), cr, ur);
+  F2 sl{fminf(ulm.x, sm.x), fminf(ulm.y, sm.y)}, sr{fmaxf(urp.x, sp.x), fmaxf(urp.y, sp.y)};
+  if (drx) sl.x = ulm.x, sr.x = ul2.x;
+  if (dry) sl.y = ulm.y, sr.y = ul2.y;
+  if (dlx) sl.x = ur2.x, sr.x = urp.x;
+  if (dly) sl.y = ur2.y, sr.y = urp.y;
+  const F2 fh_l = hl * ul, fmn_l = fma2(fh_l, ul, 0.5f * g * hl * hl);
+  const F2 fh_r = hr * ur, fmn_r = fma2(fh_r, ur, 0.5f * g * hr * hr);
+  // -min(sl, 0) and max(sr, 0)
+  const F2 a{fmaxf(-sl.x, 0.0f), fmaxf(-sl.y, 0.0f)}, b{fmaxf(sr.x, 0.0f), fmaxf(sr.y, 0.0f)};
+  const F2 gap = a + b, ab = a * b;
+  const F2 inv{rcp_near(fmaxf(gap.x, 1.0e-30f)), rcp_near(fmaxf(gap.y, 1.0e-30f))};
+  const F2 fh = fma2(b, fh_l, fma2(a, fh_r, ab * (hl - hr))) * inv;
+  const F2 fmn = fma2(b, fmn_l, fma2(a, fmn_r, ab * (fh_l - fh_r))) * inv;
+  const F2 mr = hr * (ur - sr), ml = hl * (sl - ul);
+  const F2 den_s = mr + ml, num_s = fma2(sl, mr, sr * ml), sgn = num_s * den_s;
+  const bool tx = fabsf(den_s.x) > 1.0e-12f ? sgn.x >= 0.0f : usum.x >= 0.0f;
+  const bool ty = fabsf(den_s.y) > 1.0e-12f ? sgn.y >= 0.0f : usum.y >= 0.0f;
+  const bool nx = dlx && drx, ny = dly && dry;
+  const F2 ft = fh * F2{tx ? vtl.x : vtr.x, ty ? vtl.y : vtr.y};
+  f0 = F2{nx ? 0.0f : fh.x, ny ? 0.0f : fh.y};
+  f1 = F2{nx ? 0.0f : fmn.x, ny ? 0.0f : fmn.y};
+  f2 = F2{nx ? 0.0f : ft.x, ny ? 0.0f : ft.y};
+}
+
 template <bool VOTE>
 __device__ __forceinline__ void hllc_friction(float hh, bool wet, float gdt, float n, float& hu, float& hv) {
   const float f = gdt * n * n * sqrt_near(hu * hu + hv * hv);
@@ -263,6 +298,72 @@ __device__ __forceinline__ void hllc_near(float hl, float ul, float vtl, float h
   f1 = none ? 0.0f : fmn;
   f2 = none ? 0.0f : fh * (nonneg ? vtl : vtr);
   odd |= !none & !((gap >= 0x1p-20f) & (gap <= 0x1p50f) & (dry_l | dry_r | (hs2 >= 0x1p-99f)) & sign_ok);
+}
+
+// -sqrt_rn of both halves, given them negated: the signs spare the two negations of a
+// residual correction (rounding is symmetric).
+__device__ __forceinline__ F2 neg_sqrt_rn2(F2 na) {
+  F2 y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-na.x));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-na.y));
+  const F2 nq = na * y;
+  return fma2(fma2(nq, nq, na), 0.5f * y, nq);
+}
+// hllc_near for the two faces that are the halves of its operands, the same bits. The
+// streaming kernel is bound by the instructions it issues (four in five of its cycles), and
+// half of them are adds and multiplies: in pairs, 745 -> 648 instructions a cell in stage 1
+// (2048^2, us per step: lake 290 -> 270, dam break 268 -> 246; fast dam break 190 -> 178).
+__device__ __forceinline__ void hllc_near2(F2 hl, F2 ul, F2 vtl, F2 hr, F2 ur, F2 vtr, F2& f0, F2& f1, F2& f2,
+                                           bool& odd) {
+  const float g = kG;
+  const PairOne one;
+  const bool dlx = hl.x <= kHDry, dly = hl.y <= kHDry, drx = hr.x <= kHDry, dry = hr.y <= kHDry;
+  const bool nx = dlx & drx, ny = dly & dry;
+  const F2 ncl = neg_sqrt_rn2(-g * F2{dlx ? 1.0f : hl.x, dly ? 1.0f : hl.y});
+  const F2 ncr = neg_sqrt_rn2(-g * F2{drx ? 1.0f : hr.x, dry ? 1.0f : hr.y});
+  const F2 usum = 0.5f * (ul + ur);
+  const F2 hs = 0.25f * (ul - ur) - 0.5f * (ncl + ncr);
+  const F2 hs2 = hs * hs;
+  const F2 nc_star = neg_sqrt_rn2(-g * fma2(hs2, both(0x1.a1887ap-4f), 0x1.dcb5p-38f * hs2));
+  const F2 u_star = usum - ncl + ncr;
+  const F2 ulm = ul + ncl, urp = ur - ncr, sm = u_star + nc_star, sp = u_star - nc_star;
+  const F2 ul2 = ul - (ncl + ncl), ur2 = ur + (ncr + ncr);
+  F2 sl{rmin(ulm.x, sm.x), rmin(ulm.y, sm.y)}, sr{rmax(urp.x, sp.x), rmax(urp.y, sp.y)};
+  if (drx) sl.x = ulm.x, sr.x = ul2.x;
+  if (dry) sl.y = ulm.y, sr.y = ul2.y;
+  if (dlx) sl.x = ur2.x, sr.x = urp.x;
+  if (dly) sl.y = ur2.y, sr.y = urp.y;
+  const F2 fh_l = hl * ul, fmn_l = one.add(fh_l * ul, 0.5f * g * hl * hl);
+  const F2 fh_r = hr * ur, fmn_r = one.add(fh_r * ur, 0.5f * g * hr * hr);
+  const F2 ngap = sl - sr, gap{-ngap.x, -ngap.y};
+  F2 y0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0.x) : "f"(gap.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0.y) : "f"(gap.y));
+  const F2 inv = fma2(fma2(ngap, y0, both(1.0f)), y0, y0);  // rcp_rn(gap)
+  const F2 slsr = sl * sr;
+  const F2 fh_m = one.add(one.sub(sr * fh_l, sl * fh_r), slsr * (hr - hl)) * inv;
+  const F2 fmn_m = one.add(one.sub(sr * fmn_l, sl * fmn_r), slsr * one.sub(fh_r, fh_l)) * inv;
+  const F2 ursr = ur - sr, ulsl = ul - sl;
+  const F2 den_s = one.sub(hr * ursr, hl * ulsl);
+  const F2 num_s = one.sub(sl * hr * ursr, sr * hl * ulsl);
+  auto finish = [&](float sl, float sr, float fh_l, float fh_r, float fh_m, float fmn_l, float fmn_r, float fmn_m,
+                    float den_s, float num_s, float usum, float vtl, float vtr, bool none, float& f0, float& f1,
+                    float& f2) {
+    const float fh = sl >= 0.0f ? fh_l : (sr <= 0.0f ? fh_r : fh_m);
+    const float fmn = sl >= 0.0f ? fmn_l : (sr <= 0.0f ? fmn_r : fmn_m);
+    const bool have_s = fabsf(den_s) > 1.0e-12f;
+    const bool nonneg = have_s ? (num_s == 0.0f) | ((num_s > 0.0f) == (den_s > 0.0f)) : usum >= 0.0f;
+    f0 = none ? 0.0f : fh;
+    f1 = none ? 0.0f : fmn;
+    f2 = none ? 0.0f : fh * (nonneg ? vtl : vtr);
+    return !have_s | (num_s == 0.0f) | (fabsf(num_s) > fabsf(den_s) * 0x1p-100f);
+  };
+  const bool okx = finish(sl.x, sr.x, fh_l.x, fh_r.x, fh_m.x, fmn_l.x, fmn_r.x, fmn_m.x, den_s.x, num_s.x, usum.x,
+                          vtl.x, vtr.x, nx, f0.x, f1.x, f2.x);
+  const bool oky = finish(sl.y, sr.y, fh_l.y, fh_r.y, fh_m.y, fmn_l.y, fmn_r.y, fmn_m.y, den_s.y, num_s.y, usum.y,
+                          vtl.y, vtr.y, ny, f0.y, f1.y, f2.y);
+  odd |= !nx & !((gap.x >= 0x1p-20f) & (gap.x <= 0x1p50f) & (dlx | drx | (hs2.x >= 0x1p-99f)) & okx);
+  odd |= !ny & !((gap.y >= 0x1p-20f) & (gap.y <= 0x1p50f) & (dly | dry | (hs2.y >= 0x1p-99f)) & oky);
 }
 
 template <bool VOTE>

@@ -229,8 +229,10 @@ __device__ __forceinline__ void hllc_stream_strip(const HllcParams& p, const Hll
           face_operands(wE, Quad{rx.eW, rx.zW, rx.nW, rx.tW}, kind_x, j == 0, ex, stage_x);
       float y0, y1, y2, x0, x1f, x2;
       bool odd = false;
-      hllc_near(oy.hl, oy.ul, oy.vl, oy.hr, oy.ur, oy.vr, y0, y1, y2, odd);
-      hllc_near(ox.hl, ox.ul, ox.vl, ox.hr, ox.ur, ox.vr, x0, x1f, x2, odd);
+      F2 p0, p1, p2;
+      hllc_near2(F2{oy.hl, ox.hl}, F2{oy.ul, ox.ul}, F2{oy.vl, ox.vl}, F2{oy.hr, ox.hr}, F2{oy.ur, ox.ur},
+                 F2{oy.vr, ox.vr}, p0, p1, p2, odd);
+      y0 = p0.x, y1 = p1.x, y2 = p2.x, x0 = p0.y, x1f = p1.y, x2 = p2.y;
 #if !defined(RB_FAST_MATH)
       if (__any_sync(kFullWarp, odd)) {
         hllc_flux_any(oy.hl, oy.ul, oy.vl, oy.hr, oy.ur, oy.vr, y0, y1, y2);

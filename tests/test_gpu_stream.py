@@ -108,23 +108,23 @@ def _hllc(ny, nx, seed, **more):
 
 STAGES = {"east": [(0.0, 1.4), (1.0e4, 0.9)], "north": [(0.0, 0.8), (1.0e4, 1.3)]}
 
-# 1540 x 1300: a last strip with all 26 columns; 1001 x 2003: one column in the last strip;
-# 90 x 23000: a flat domain with a short last chunk.
+# 2308 x 1300: a last strip with all 26 columns; 1501 x 2003: one column in the last strip;
+# 135 x 23000: a flat domain with a short last chunk.
 HLLC_CASES = {
-    "closed": lambda: _hllc(1540, 1300, 1),
-    "open_rain": lambda: _hllc(1001, 2003, 2, compensated=True, rain=50.0 * MM_H, boundaries=ALL_OPEN),
-    "stage_plain_rain": lambda: _hllc(90, 23000, 3, rain=50.0 * MM_H, stage_curves=STAGES,
+    "closed": lambda: _hllc(2308, 1300, 1),
+    "open_rain": lambda: _hllc(1501, 2003, 2, compensated=True, rain=50.0 * MM_H, boundaries=ALL_OPEN),
+    "stage_plain_rain": lambda: _hllc(135, 23000, 3, rain=50.0 * MM_H, stage_curves=STAGES,
                                       boundaries={"east": "fixed_stage", "north": "fixed_stage", "west": "open"}),
-    "field_infil": lambda: _hllc(1001, 2003, 4, compensated=True, boundaries={"south": "open"},
-                                 rain_field=np.full((1001, 2003), 40.0 * MM_H, np.float32),
-                                 infil=np.full((1001, 2003), 2000.0 * MM_H, np.float32)),
+    "field_infil": lambda: _hllc(1501, 2003, 4, compensated=True, boundaries={"south": "open"},
+                                 rain_field=np.full((1501, 2003), 40.0 * MM_H, np.float32),
+                                 infil=np.full((1501, 2003), 2000.0 * MM_H, np.float32)),
     # still water with islands: zero velocities, zero contact speeds, rest at the shore
-    "still": lambda: _hllc(1540, 1300, 5, hu0=np.zeros((1540, 1300), np.float32),
-                           hv0=np.zeros((1540, 1300), np.float32)),
+    "still": lambda: _hllc(2308, 1300, 5, hu0=np.zeros((2308, 1300), np.float32),
+                           hv0=np.zeros((2308, 1300), np.float32)),
     # momenta down to the subnormals and depths up to 1e5: outside the quick divisions
-    "odd_operands": lambda: _hllc(1001, 2003, 6, hu0=np.full((1001, 2003), 1e-39, np.float32),
-                                  hv0=np.full((1001, 2003), -1e-25, np.float32), bed=np.zeros((1001, 2003), np.float32),
-                                  depth=np.logspace(-6, 5, 2003, dtype=np.float32)[None, :].repeat(1001, 0)),
+    "odd_operands": lambda: _hllc(1501, 2003, 6, hu0=np.full((1501, 2003), 1e-39, np.float32),
+                                  hv0=np.full((1501, 2003), -1e-25, np.float32), bed=np.zeros((1501, 2003), np.float32),
+                                  depth=np.logspace(-6, 5, 2003, dtype=np.float32)[None, :].repeat(1501, 0)),
 }  # fmt: skip
 
 
@@ -133,8 +133,8 @@ NAN_CASES = {
     "li": lambda: _li(1429, 1400, 10, steps=3, depth=_with_nan(
         np.full((1429, 1400), 0.3, np.float32), [(700, 700), (1000, 27), (1001, 28), (0, 5), (1428, 1399)])),
     # depths and momenta that are not numbers
-    "hllc": lambda: _hllc(1540, 1300, 7, steps=2, hu0=_with_nan(np.ones((1540, 1300), np.float32), [(800, 800), (51, 26)]),
-                         depth=_with_nan(np.ones((1540, 1300), np.float32), [(700, 700), (50, 25), (0, 4), (1539, 9)])),
+    "hllc": lambda: _hllc(2308, 1300, 7, steps=2, hu0=_with_nan(np.ones((2308, 1300), np.float32), [(800, 800), (51, 26)]),
+                         depth=_with_nan(np.ones((2308, 1300), np.float32), [(700, 700), (50, 25), (0, 4), (2307, 9)])),
 }  # fmt: skip
 
 
