@@ -41,6 +41,7 @@
 namespace rb {
 RB_ARITH_BEGIN
 
+#include "pair.cuh"
 #include "warp_stream.cuh"
 
 #if defined(RB_FAST_MATH)

@@ -42,6 +42,61 @@ __device__ __forceinline__ void li_faces(const float (&qo)[NF], const float (&el
   }
 }
 #else
+// The steps of div_rn and pow73_mid on both halves, the same bits (the power compared with
+// rb_pow73f on all 268 435 456 floats of [2^-12, 2^20)): the x-face and the y-face of a
+// row in one instruction each, 97.9 -> 91.6 us per 2048^2 step. The quotients are
+// negated until their sign is set, which spares the negations of the residuals.
+__device__ __forceinline__ F2 div_rn_by2(F2 a, F2 b, F2 ny) {  // ny = -1 / b, rounded once
+  const F2 nq0 = a * ny;
+  const F2 nq = fma2(fma2(b, nq0, a), ny, nq0);
+  return F2{__uint_as_float((__float_as_uint(nq.x) & 0x7fffffffu) | (__float_as_uint(a.x) & 0x80000000u)),
+            __uint_as_float((__float_as_uint(nq.y) & 0x7fffffffu) | (__float_as_uint(a.y) & 0x80000000u))};
+}
+__device__ __forceinline__ F2 neg_rcp_rn2(F2 b) {
+  F2 y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-b.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-b.y));
+  return fma2(fma2(b, y, both(1.0f)), y, y);
+}
+__device__ __forceinline__ F2 pow73_mid2(F2 x, const PairOne& one) {
+  int kx, ky, qx, qy, rx, ry;
+  F2 m, tf;
+  auto split = [](float x, int& k, int& q, int& r, float& m, float& tf) {
+    const unsigned b = __float_as_uint(x);
+    k = (int)(b >> 23) - 115;
+    q = (k * 43) >> 7;
+    r = k - 3 * q;
+    const unsigned mb = (b & 0x007fffffu) | 0x3f800000u;
+    m = __uint_as_float(mb);
+    tf = __uint_as_float(mb + ((unsigned)r << 23));
+  };
+  split(x.x, kx, qx, rx, m.x, tf.x);
+  split(x.y, ky, qy, ry, m.y, tf.y);
+  F2 w = one.add(both(-0.0488736666738987f) * m, both(0.3129411041736603f));
+  w = one.add(w * m, both(-0.8028873205184937f));
+  w = one.add(w * m, both(1.5385289192199707f));
+  auto scale = [](int r) { return r == 0 ? 1.0f : (r == 1 ? 0.7937005162239075f : 0.6299605369567871f); };
+  w = w * F2{scale(rx), scale(ry)};
+  w = one.add(w, w * (one.sub(both(1.0f), tf * (w * w * w)) * both(0.333333343f)));
+  const F2 t1 = m - both(1.0f);
+  F2 l = one.add(both(0.04392862692475319f) * t1, both(-0.18983244895935059f));
+  l = one.add(l * t1, both(0.4115614891052246f));
+  l = one.add(l * t1, both(-0.7072534561157227f));
+  l = one.add(l * t1, both(1.4415920972824097f));
+  l = one.add(l * t1, both(1.4390930118679535e-05f));
+  auto ef = [](int k) { return __uint_as_float(0x4b000000u + (unsigned)k) - 8388620.0f; };
+  const F2 ln = (F2{ef(kx), ef(ky)} + l) * both(0.693147182f);
+  auto finish = [](float tf, float wf, float ln, int q) {
+    const double t = (double)tf;
+    double wd = (double)wf;
+    wd = wd + wd * ((1.0 - t * ((wd * wd) * wd)) * 0.3333333333333333);
+    const double u = RB_DELTA_73 * (double)ln;
+    const double v = ((t * t) * (t * (wd * wd))) * ((1.0 - u) + 0.5 * (u * u));
+    return __uint_as_float(__float_as_uint((float)v) + ((unsigned)(7 * (q - 4)) << 23));
+  };
+  return F2{finish(tf.x, w.x, ln.x, qx), finish(tf.y, w.y, ln.y, qy)};
+}
+
 // Exact arithmetic, without a branch per face: the divisions are div_rn (rb_common.cuh)
 // on operands inside its range, and a warp with a face outside it takes the reference's
 // expressions face by face. A friction numerator f below 2^-60 cannot lift the
@@ -51,28 +106,31 @@ template <int NF>
 __device__ __forceinline__ void li_faces(const float (&qo)[NF], const float (&el)[NF], const float (&er)[NF],
                                          const float (&h)[NF], const float (&n)[NF], const bool (&on)[NF],
                                          const LiFaceConst& c, float (&q)[NF]) {
-  float num[NF], f[NF], de[NF];
+  static_assert(NF == 2, "the faces are the halves of packed pairs");
+  const PairOne one;
+  const F2 ho{h[0], h[1]}, no{n[0], n[1]}, qp{qo[0], qo[1]};
+  const F2 de = F2{er[0], er[1]} - F2{el[0], el[1]};
+  const F2 num = one.sub(qp, kG * ho * both(c.dt) * div_rn_by2(de, both(c.dx), both(-c.rdx)));
+  const F2 f = c.gdt * no * no * F2{fabsf(qo[0]), fabsf(qo[1])};
   bool wet[NF], need = false, odd = c.rdx == 0.0f;
-#pragma unroll
-  for (int i = 0; i < NF; i++) {
-    wet[i] = on[i] & !(h[i] < kHDry);
-    de[i] = er[i] - el[i];
-    const float slope = div_rn_by(de[i], c.dx, c.rdx);
-    num[i] = qo[i] - kG * h[i] * c.dt * slope;
-    f[i] = c.gdt * n[i] * n[i] * fabsf(qo[i]);
-    const bool small = div_rn_small_ok(de[i]) & div_rn_small_ok(num[i]);
-    const bool large = !(fmaxf(fabsf(de[i]), fabsf(num[i])) > 0x1p60f) & (h[i] <= 0x1p19f) & (f[i] <= 0x1p40f);
-    odd |= wet[i] & !(small & large);
-    need |= wet[i] & (f[i] >= 0x1p-60f);
-    q[i] = wet[i] ? num[i] : 0.0f;
-  }
+  auto check = [&](bool on, float h, float de, float num, float f, bool& wet, float& q) {
+    wet = on & !(h < kHDry);
+    const bool small = div_rn_small_ok(de) & div_rn_small_ok(num);
+    const bool large = !(fmaxf(fabsf(de), fabsf(num)) > 0x1p60f) & (h <= 0x1p19f) & (f <= 0x1p40f);
+    odd |= wet & !(small & large);
+    need |= wet & (f >= 0x1p-60f);
+    q = wet ? num : 0.0f;
+  };
+  check(on[0], h[0], de.x, num.x, f.x, wet[0], q[0]);
+  check(on[1], h[1], de.y, num.y, f.y, wet[1], q[1]);
   if (__any_sync(kFullWarp, need)) {
-#pragma unroll
-    for (int i = 0; i < NF; i++) {
-      const float den = 1.0f + div_rn(f[i], pow73_mid(wet[i] ? h[i] : 1.0f));
-      odd |= wet[i] & !(den <= 0x1p20f);
-      q[i] = wet[i] ? div_rn(num[i], den) : 0.0f;
-    }
+    const F2 p = pow73_mid2(F2{wet[0] ? h[0] : 1.0f, wet[1] ? h[1] : 1.0f}, one);
+    const F2 ratio = div_rn_by2(f, p, neg_rcp_rn2(p));
+    const F2 den = both(1.0f) + ratio;
+    odd |= (wet[0] & !(den.x <= 0x1p20f)) | (wet[1] & !(den.y <= 0x1p20f));
+    const F2 v = div_rn_by2(num, den, neg_rcp_rn2(den));
+    q[0] = wet[0] ? v.x : 0.0f;
+    q[1] = wet[1] ? v.y : 0.0f;
   }
   if (__any_sync(kFullWarp, odd)) {
 #pragma unroll 1
