@@ -281,13 +281,15 @@ int rb_ensemble_read(const rb_ensemble_layout *L, void *ens, rb_clock_state *out
  * where a row is not a multiple of 16 bytes; 8 does the same with one persistent block
  * per resident slot that prefetches the halo of its next tile). Every variant computes bit-identical
  * results; this is a speed knob only, read at each launch (a captured graph keeps
- * the variant it was captured with). The library starts with the variant measured
- * fastest on B200 (6: 32 x 32 tiles, 640 threads). */
+ * the variant it was captured with). The library starts with 6, which picks by the
+ * domain's size what measured fastest on B200: 16 x 16, 32 x 16 or 32 x 32 tiles, or a
+ * row-streaming kernel. */
 int rb_hllc_set_kernel_variant(int32_t variant);
 int rb_hllc_kernel_variants(int32_t *count);
 /* The same for the local-inertial step (tile 32 x 16, 32 x 32, 64 x 16, 32 x 8, and
  * 32 x 16 held to 48 registers; a state with sub-grid channels always uses 32 x 16).
- * The library starts with variant 1 (32 x 32 tiles, 512 threads). */
+ * The library starts with 1, which picks by the domain's size: 16 x 16 or 32 x 32 tiles,
+ * or a row-streaming kernel. */
 int rb_li_set_kernel_variant(int32_t variant);
 int rb_li_kernel_variants(int32_t *count);
 

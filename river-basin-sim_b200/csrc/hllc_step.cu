@@ -20,6 +20,8 @@
 // own faces. Stage 1 writes U1 = (h1, hu1, hv1) to workspace buffers; stage 2
 // reads U1 with the halo and U^n on the tile and writes U^{n+1} to the other
 // buffer of the caller's double-buffered (h, hu, hv).
+//
+// Large domains are stepped by the row-streaming form of hllc_stream.cuh instead.
 #include <cuda.h>  // CUtensorMap and its encoder's signature (reached through the runtime)
 
 #include <algorithm>
@@ -1443,16 +1445,15 @@ static cudaError_t launch_hllc_tma(const HllcParams& p, int stage, cudaStream_t 
 }
 
 // Kernel variants of the single-domain stage: tile, block size, faces per work item,
-// load batching. All compute the same bits; they differ only in speed. The default
-// (6: 32 x 32 tiles, 640 threads, two blocks and 40 warps per SM, 44-48 registers)
-// is the fastest measured on B200: 0.316 ms per 2048 x 2048 dam-break step against
-// 0.326 for 512 threads, 0.337 for 576, 0.323 for 608, 0.328 for 768 and 0.348 for
-// 800 (which spills at its 40-register bound). The 2380 face work items of a tile
-// fill 3.7 passes of 640 threads against 4.6 of 512. Staging interior tiles with
-// tensor-memory copies measures 0.319 ms (7: one tile a block) and 0.360 ms (8: one
-// resident block of 512 threads per slot walking the tiles and prefetching the next
-// one's halo, against 0.330 for the same block as a grid of tiles): the copies free no
-// issue slots the tile needs, and a static walk leaves SMs idle at the end.
+// load batching. All compute the same bits; they differ only in speed. The default (6)
+// chooses by the domain's size (hllc_default_tile, hllc_stream_takes); its 32 x 32 tiles
+// have 640 threads, two blocks and 40 warps per SM at 44-48 registers: fewer leave the
+// 2380 face work items of a tile an emptier last pass (3.7 passes of 640 threads, 4.6 of
+// 512), more spill. Staging interior tiles with tensor-memory copies is slower (7: one
+// tile a block, by 1 %; 8: one resident block of 512 threads per slot walking the tiles
+// and prefetching the next one's halo, by 9 % against the same block as a grid of tiles):
+// the copies free no issue slots the tile needs, and a static walk leaves SMs idle at the
+// end.
 struct HllcKernelVariant {
   int tx, ty, nt, fu, lp;
 };

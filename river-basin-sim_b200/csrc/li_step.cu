@@ -26,6 +26,9 @@
 // the water column instead of h for the next dt. The unarmed instantiation does
 // none of it.
 //
+// Large domains are stepped by the row-streaming form of li_stream.cuh instead, which
+// computes each halo cell and face once per strip and keeps rows in registers.
+//
 // Per-cell HBM traffic (compulsory): read h, z, n, qx, qy, write h, qx, qy (32 B),
 // + h_comp read/write (8 B) when compensated rain is armed, + rain field / infil
 // reads (4 B each), + d50 and the four transport accumulators (36 B) when
@@ -704,9 +707,9 @@ static bool li_small(const LiParams& p) {
 }
 
 // Tile variants of the single-domain step (sub-grid channels always use 32 x 16);
-// all compute the same bits. The default is the fastest measured on B200 for the
-// 2048^2 and 4096^2 rain-on-grid steps (ms per 2048^2 step: 0.158, 0.142, 0.145,
-// 0.208, 0.149 for variants 0..4).
+// all compute the same bits. The default (1) chooses by the domain's size: 16 x 16
+// (li_small), 32 x 32 or the streaming kernel (li_stream_takes). Of the tiles 32 x 32 were
+// the fastest on B200 on the 2048^2 and 4096^2 rain-on-grid steps.
 struct LiKernelVariant {
   int tx, ty, nt;
 };

@@ -3,7 +3,7 @@
 Requests (scheme, grid side, horizon, seeded synthetic terrain, optional Exner
 morphology) arrive over wall-clock time. The server admits them in arrival order
 while the HBM they need fits the budget, keeps every admitted solve resident, and
-steps all of them together as one ``Ensemble`` (one persistent kernel per scheme
+steps all of them together as one ``Ensemble`` (one kernel per scheme
 over the members' tiles, the single-domain kernels for members large enough to fill
 the GPU alone; each member on its own device clock). Between graph
 replays it retires finished solves (their results at once; a finished member stays
