@@ -61,12 +61,12 @@ DT_MAX = 30.0
 T_END = 30.0  # simulated horizon of the dam-break configuration
 BYTES_PER_CELL_STEP = 32  # read h, hu, hv, z, n (20 B) + write h, hu, hv (12 B)
 # DRAM bytes (read + write) of one step's two stage launches in one ncu capture of this
-# workload (--set full, 2048^2 dam break, fast build, stage 1 + stage 2): 87.2 MB +
-# 165.5 MB (the exact build: 88.3 + 163.5 MB).
-NCU_DRAM_BYTES_PER_STEP = 252.7e6
+# workload (2048^2 dam break, streaming kernels, fast build, stage 1 + stage 2): 83.3 MB +
+# 178.0 MB (the exact build: 83.4 + 175.6 MB).
+NCU_DRAM_BYTES_PER_STEP = 261.4e6
 # The stage kernels are issue-bound: share of issue slots busy in the same capture
-# (fast build: stage 1 83.4 %, stage 2 82.4 %; exact: 84.8 %, 84.3 %).
-NCU_ISSUE_ACTIVE = (0.834, 0.824)
+# (fast build: stage 1 72.5 %, stage 2 68.7 %; exact: 73.0 %, 71.9 %).
+NCU_ISSUE_ACTIVE = (0.725, 0.687)
 WORKLOAD = "hllc_dambreak_2048x2048"
 BUILDS = {
     "exact": "exact: one IEEE rounding per operation in the reference's order, bit-identical to the oracle",
@@ -430,7 +430,7 @@ def main(argv=None) -> int:
                          "issue_bound": {"issue_slots_busy_stage1": NCU_ISSUE_ACTIVE[0],
                                          "issue_slots_busy_stage2": NCU_ISSUE_ACTIVE[1],
                                          "source": "the same ncu capture"},
-                         "kernel": "hllc_stage_kernel stage 1 + stage 2 (one SSP-RK2 step)",
+                         "kernel": "hllc_stream_kernel stage 1 + stage 2 (one SSP-RK2 step)",
                          "bytes_per_cell_step": BYTES_PER_CELL_STEP,
                          "launched_one_by_one": {"stage_pair_ms_mean": mean_kernel_ms,
                                                  "stage1_ms_mean": statistics.mean(stage1_ms),

@@ -228,9 +228,9 @@ def li_rain_2048(args, legs: bool = True):
     _kernel_roofline(st, "local_inertial", max(args.warmup, 1), 40, rain_rate=RAIN_50_MM_H)  # warm-up steps
     roof = _kernel_roofline(st, "local_inertial", args.steps, 40, rain_rate=RAIN_50_MM_H)
     # DRAM bytes read + written by one launch in an ncu capture of this workload (fast
-    # build): 100.8 + 30.9 MB against 167.8 MB algorithmic (L2 keeps part of the last step)
-    roof["traffic"] = 131.6e6
-    roof["traffic_note"] = "one launch, ncu --set full capture of this workload (fast build)"
+    # build): 111.9 + 28.9 MB against 167.8 MB algorithmic (L2 keeps part of the last step)
+    roof["traffic"] = 140.8e6
+    roof["traffic_note"] = "one launch, ncu capture of this workload (fast build)"
     del st
     out = {"workload": "li_rain_2048", "metric": "Gcell-updates/s", "value": roof["gcell_per_s_step"],
            "steps": args.steps, "warmup": args.warmup, "roofline": roof,

@@ -1473,6 +1473,11 @@ int hllc_kernel_variant_count() { return kNumHllcVariants; }
 // Set every variant's shared-memory opt-in on the current device, outside any
 // stream capture (called by the non-capturable set-up entry points).
 void hllc_prepare_device() {
+  static std::atomic<unsigned long long> prepared{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (prepared.load() & bit) return;
   prepare_hllc<32, 16, 256, 1, 0>();
   prepare_hllc<32, 16, 256, 1, 1>();
   prepare_hllc<32, 16, 256, 3, 1>();
@@ -1487,6 +1492,7 @@ void hllc_prepare_device() {
 #if !defined(RB_FAST_MATH)
   fast::hllc_prepare_device();
 #endif
+  prepared.fetch_or(bit);
 }
 #if !defined(RB_FAST_MATH)
 bool hllc_set_kernel_variant(int v) {
