@@ -45,37 +45,63 @@ inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 rb::WsHeader* header(void* ws) { return static_cast<rb::WsHeader*>(ws); }
 
 // Where a reduction's one word comes back: a mapped, page-locked host word that the kernel
-// writes itself, one per host thread (given back when the thread ends), which saves the
-// copy's launch and its staging; or, where none can be had, the workspace's word and a copy.
-// The caller synchronises before it reads, so a thread has one in flight at most.
-struct MappedWord {
+// writes itself, which saves the copy's launch and its staging; or, where none can be had,
+// the workspace's word and a copy. A call holds a word until it has synchronised. The words
+// are one 16 KB allocation for the process, made when its first workspace is set up (it
+// takes milliseconds, more than the steps it would delay).
+struct MappedWords {
+  static constexpr int kWords = 256, kStride = 16;  // a cache line apart
   unsigned int* host = nullptr;
-  MappedWord() {
+  std::atomic<unsigned long long> busy[kWords / 64] = {};
+  MappedWords() {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // another thread may be capturing
+    const bool exchanged = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
     void* p = nullptr;
-    if (cudaHostAlloc(&p, sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
+    if (cudaHostAlloc(&p, kWords * kStride * sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped) ==
+        cudaSuccess)
       host = static_cast<unsigned int*>(p);
     else
       cudaGetLastError();
+    if (exchanged) cudaThreadExchangeStreamCaptureMode(&mode);
   }
-  ~MappedWord() {
-    if (host != nullptr) cudaFreeHost(host);
+  int take() {
+    for (int w = 0; w < kWords / 64 && host != nullptr; w++) {
+      unsigned long long taken = busy[w].load();
+      while (taken != ~0ull) {
+        const int bit = __builtin_ctzll(~taken);
+        taken = busy[w].fetch_or(1ull << bit);
+        if (!(taken >> bit & 1)) return 64 * w + bit;
+      }
+    }
+    return -1;
   }
+  void give(int k) { busy[k / 64].fetch_and(~(1ull << (k % 64))); }
 };
+MappedWords& mapped_words() {
+  static MappedWords* words = new MappedWords;  // for the life of the process
+  return *words;
+}
 
 struct ResultWord {
   unsigned int* device;
   unsigned int* mapped = nullptr;
-  explicit ResultWord(rb::WsHeader* h) : device(&h->red_key) {
-    static thread_local MappedWord word;
+  int slot;
+  explicit ResultWord(rb::WsHeader* h) : device(&h->red_key), slot(mapped_words().take()) {
+    if (slot < 0) return;
+    unsigned int* word = mapped_words().host + slot * MappedWords::kStride;
     void* d = nullptr;
-    if (word.host == nullptr) return;
-    if (cudaHostGetDevicePointer(&d, word.host, 0) == cudaSuccess) {
-      mapped = word.host;
+    if (cudaHostGetDevicePointer(&d, word, 0) == cudaSuccess) {
+      mapped = word;
       device = static_cast<unsigned int*>(d);
     } else {
       cudaGetLastError();
     }
   }
+  ~ResultWord() {
+    if (slot >= 0) mapped_words().give(slot);
+  }
+  ResultWord(const ResultWord&) = delete;
+  ResultWord& operator=(const ResultWord&) = delete;
   int read(float* out, cudaStream_t s, const char* who) const {
     unsigned int key = 0;
     if (mapped == nullptr) RB_CUDA(cudaMemcpyAsync(&key, device, sizeof key, cudaMemcpyDeviceToHost, s), who);
@@ -271,6 +297,7 @@ int rb_workspace_init(void* ws, size_t bytes, void* stream) {
   if (ws == nullptr || bytes < rb::WS_LEDGER) return fail(RB_ERR_ARG, "rb_workspace_init: workspace too small");
   RB_CUDA(cudaMemsetAsync(ws, 0, bytes, (cudaStream_t)stream), "rb_workspace_init");
   rb::hllc_prepare_device();  // kernel attributes, before any stream capture
+  mapped_words();
   return RB_OK;
 }
 

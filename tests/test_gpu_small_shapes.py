@@ -63,7 +63,7 @@ def test_dt_is_that_of_the_largest_depth_wherever_it_is(n):
 
 
 def test_dt_from_several_threads_and_streams():
-    """Each thread has its own result word: eight of them, on their own streams, read the dt
+    """A call holds a result word of its own: eight threads, on their own streams, read the dt
     of their own state every time."""
     from rbsim.schemes import local_inertial as li
 
