@@ -403,7 +403,7 @@ __device__ __forceinline__ void hllc_stream_block(const HllcParams& p, int strip
 
 // One warp a block (no sibling to wait for at the end), 16 resident per SM: at 20 and 24
 // (96 and 80 registers) the schedulers have no more to issue and the spills show (2048^2
-// dam break, us per step, fast / exact: 189.7 / 270 for 16, 198.8 / 296 for 20, 209.9 / 308
+// dam break, faces one by one, us per step, fast / exact: 189.7 / 270 for 16, 198.8 / 296 for 20, 209.9 / 308
 // for 24).
 constexpr int kHllcStreamWarps = 16;
 template <int STAGE, int SRC>
@@ -426,13 +426,14 @@ static cudaError_t launch_hllc_stream(const HllcParams& p, int stage, cudaStream
 // Whether the streaming kernel takes this domain (with hllc_stream_fits). Below these sizes
 // the 32 x 32 tiles are as fast or faster: a warp walks its rows one after another, and a
 // small domain has too few warps to hide that; on a narrow one the strips at the west and
-// east edge, which check bounds, are too many (dam breaks, us per step, tiles / streaming
-// -- fast: 1024^2 72.0 / 73.8, 1448^2 138 / 114, 2048^2 265 / 190, 4096^2 1011 / 633; exact:
-// 1448^2 161 / 162, 2048^2 306 / 268, 4096^2 1180 / 912; lake, 2600 x 480 fast 91.7 / 98.7).
+// east edge, which check bounds, are too many (us per step, tiles / streaming -- fast dam
+// breaks: 1024^2 65.6 / 67.4, 1200^2 87.8 / 82.7, 2048^2 265 / 178; exact lakes: 1024^2 87 /
+// 100, 1200^2 116 / 122, 1448^2 164 / 157, 2600 x 800 161 / 163, 1600^2 198 / 185; exact
+// dam break, 2048^2 306 / 246).
 #if defined(RB_FAST_MATH)
 constexpr long long kHllcStreamCells = 1500000;
 #else
-constexpr long long kHllcStreamCells = 3000000;
+constexpr long long kHllcStreamCells = 2300000;
 #endif
 static bool hllc_stream_takes(const HllcParams& p) {
   return (long long)p.ny * p.nx >= kHllcStreamCells && p.nx >= 30 * kHllcStreamCols && hllc_stream_fits(p.ny, p.nx);
