@@ -302,15 +302,6 @@ __device__ __forceinline__ void hllc_near(float hl, float ul, float vtl, float h
   odd |= !none & !((gap >= 0x1p-20f) & (gap <= 0x1p50f) & (dry_l | dry_r | (hs2 >= 0x1p-99f)) & sign_ok);
 }
 
-// -sqrt_rn of both halves, given them negated: the signs spare the two negations of a
-// residual correction (rounding is symmetric).
-__device__ __forceinline__ F2 neg_sqrt_rn2(F2 na) {
-  F2 y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-na.x));
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-na.y));
-  const F2 nq = na * y;
-  return fma2(fma2(nq, nq, na), 0.5f * y, nq);
-}
 // hllc_near for the two faces that are the halves of its operands, the same bits. The
 // streaming kernel is bound by the instructions it issues (four in five of its cycles), and
 // half of them are adds and multiplies: in pairs, 745 -> 648 instructions a cell in stage 1

@@ -59,24 +59,24 @@ __device__ __forceinline__ float div_if(bool use, float x, float y) { return use
 __device__ __forceinline__ float div_in_branch(float x, float y) { return x / y; }
 // x / g
 __device__ __forceinline__ float div_g(float x) { return x * (1.0f / kG); }
-// x * rcp_near(y) has the bits of the full-range division x / y above for |y| in
-// [2^-60, 2^60] (three billion random pairs compared), without its range scaling; a sum
-// that follows contracts with it as it does with the division's last product.
+// A quotient as x times the reciprocal unit's approximation: within 2^-22 of x / y for
+// |y| in [2^-60, 2^60] (the unit is documented to an ulp, the product rounds once more).
 __device__ __forceinline__ float rcp_near(float y) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
   return r;
 }
-// The approximate square root, flushing subnormals.
+// The square-root unit: within 2^-23 for a normal x (as documented), 0 for a subnormal.
 __device__ __forceinline__ float sqrt_near(float x) {
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-// h^(7/3) for a normal h >= H_DRY: __powf's bits without its handling of subnormals. The
-// maximum changes nothing there (the power is above 2^-24); it keeps the assembler from
-// folding a reciprocal of the result into an exponential of the negated argument, which
-// rounds differently.
+// h^(7/3) for h in [H_DRY, 2^20] as 2^(p log2 h) on the logarithm and exponential units.
+// With their documented errors (2^-22 of max(1, |log2 h|), and 2 ulp) the relative error
+// is below ln 2 (p 2^-22 max(1, |log2 h|) + 2^-24 |p log2 h|) + 2^-22 + 2^-24. The power
+// is above 2^-24 there, so that the maximum changes no value; without it the power and the
+// reciprocal that callers take of it came out an ulp apart from the two taken one by one.
 __device__ __forceinline__ float pow73_near(float h) {
   float l, e;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(h));
@@ -137,9 +137,12 @@ __device__ __forceinline__ float div_in_branch(float x, float y) {
 // RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990: with y the correctly
 // rounded 1 / b and q0 within an ulp of a / b, RN(q0 + y RN(a - b q0)) is the correctly
 // rounded quotient). One Newton step on this GPU's approximation gives that y for every
-// b in [2^-24, 2^64] (all 738 197 505 of them compared with __frcp_rn). Neither quotient
-// nor residual may underflow: |a| in [2^-60, 2^60] or a = 0 (div_rn_small_ok checks the
-// lower end) with b <= 2^24. Outside, the result is unspecified; a NaN a gives NaN.
+// b in [2^-24, 2^64] (tests/test_gpu_arith_sweep.py compares all of them, and the other
+// ranges named here, with the IEEE operations). Over the same b the quotient is exact in
+// this sense for |a| in [2^-60, 2^60] or a = 0 (div_rn_small_ok checks the lower end): it
+// stays above 2^-124, and its residual, a multiple of 2^-107 or more, does not underflow.
+// Outside, the result is unspecified, but for b >= 2^-24 never above 2^-35 where |a| <
+// 2^-60; a NaN a gives NaN.
 __device__ __forceinline__ bool div_rn_small_ok(float a) { return (a == 0.0f) | !(fabsf(a) < 0x1p-60f); }
 // a / b given y, the correctly rounded 1 / b, for b > 0: the sign is the dividend's, also
 // that of a zero.
@@ -156,7 +159,7 @@ __device__ __forceinline__ float rcp_rn(float b) {  // the correctly rounded 1 /
 __device__ __forceinline__ float div_rn(float a, float b) { return div_rn_by(a, b, rcp_rn(b)); }
 
 // The IEEE square root for a in [2^-100, 2^100]: Markstein's residual correction of
-// a * rsqrt(a) (same paper), compared with __fsqrt_rn on all 1 677 721 601 of them.
+// a * rsqrt(a) (same paper).
 __device__ __forceinline__ float sqrt_rn(float a) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
