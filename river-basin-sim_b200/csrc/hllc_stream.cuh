@@ -365,6 +365,9 @@ __device__ __forceinline__ void hllc_stream_strip(const HllcParams& p, const Hll
 #pragma unroll 1
 #endif
   for (; r <= i1 + 2; r++) iterate(r, std::true_type{});
+  // the copy ahead of the last row: nothing may land in the next block's shared memory.
+  // (Not starting it instead: 2048^2 lake 1.1 % slower, fast dam break 1.5 % faster.)
+  cp_async_wait<0>();
   if (!EDGE && !own) smax = 0.0f, bad = false;
 }
 

@@ -350,6 +350,9 @@ __device__ __forceinline__ void li_stream_strip(const LiParams& p, const LiStepS
 #endif
     for (; r <= i1; r++) iterate(r, std::true_type{});
     iterate(r, std::false_type{});
+    // the copy ahead of the last row: nothing may land in the next block's shared memory.
+    // (Not starting it instead: the 8192^2 reach 0.5 % slower.)
+    cp_async_wait<0>();
     if (!own) hmax = 0.0f, bad = false;
   }
 }
