@@ -260,7 +260,8 @@ static void ens_regroup(EnsRoute<Params>& r, const std::vector<rb::DevClock>& cl
   long long cells = 0;
   for (size_t i = 0; i < r.rows.size(); i++) {
     const rb::DevClock& c = clocks[r.row_dom[i]];
-    if (c.t < c.t_target && c.steps < c.max_steps) cells += (long long)r.rows[i].ny * r.rows[i].nx;
+    if (c.t < c.t_target - rb::kEpsT && c.steps < c.max_steps)  // as the plan decides it
+      cells += (long long)r.rows[i].ny * r.rows[i].nx;
   }
   r.grouped = !r.rows.empty() && cells >= r.cells_min;
 }
@@ -745,6 +746,14 @@ struct EnsSolo {
 static std::mutex g_ens_solo_mu;
 static std::unordered_map<const void*, EnsSolo> g_ens_solo;
 
+static void ens_regroup(const void* ens, const std::vector<rb::DevClock>& clocks) {
+  std::lock_guard<std::mutex> lock(g_ens_solo_mu);
+  auto it = g_ens_solo.find(ens);
+  if (it == g_ens_solo.end()) return;
+  ens_regroup(it->second.li, clocks);
+  ens_regroup(it->second.hllc, clocks);
+}
+
 int rb_ensemble_layout_make(int32_t ndom, const int32_t* scheme, const int32_t* ny, const int32_t* nx,
                             int32_t li_variant, int32_t hllc_variant, rb_ensemble_layout* out) {
   if (ndom < 1 || !scheme || !ny || !nx || !out) return fail(RB_ERR_ARG, "rb_ensemble_layout_make: bad argument");
@@ -929,15 +938,19 @@ int rb_ensemble_set_targets(const rb_ensemble_layout* L, void* ens, const double
   RB_CUDA(cudaMemcpyAsync(dt_t, t_target, (size_t)L->ndom * sizeof(double), cudaMemcpyHostToDevice, s), "targets");
   RB_CUDA(cudaMemcpyAsync(dm, max_steps, (size_t)L->ndom * sizeof(int32_t), cudaMemcpyHostToDevice, s), "targets");
   RB_CUDA(rb::clock_target_many_launch((rb::DevClock*)(base + L->off_clocks), L->ndom, dt_t, dm, s), "targets");
-  RB_CUDA(cudaStreamSynchronize(s), "rb_ensemble_set_targets sync");
+  bool groups = false;  // the clocks decide only whether domains are grouped
   {
     std::lock_guard<std::mutex> lock(g_ens_solo_mu);
     auto it = g_ens_solo.find(ens);
-    if (it != g_ens_solo.end()) {
-      it->second.li.grouped = !it->second.li.rows.empty();
-      it->second.hllc.grouped = !it->second.hllc.rows.empty();
-    }
+    groups = it != g_ens_solo.end() && !(it->second.li.rows.empty() && it->second.hllc.rows.empty());
   }
+  std::vector<rb::DevClock> hc(groups ? L->ndom : 0);
+  if (groups)
+    RB_CUDA(cudaMemcpyAsync(hc.data(), base + L->off_clocks, hc.size() * sizeof(rb::DevClock), cudaMemcpyDeviceToHost,
+                            s),
+            "targets");
+  RB_CUDA(cudaStreamSynchronize(s), "rb_ensemble_set_targets sync");
+  if (groups) ens_regroup(ens, hc);
   return RB_OK;
 }
 
@@ -993,14 +1006,7 @@ int rb_ensemble_read(const rb_ensemble_layout* L, void* ens, rb_clock_state* out
   std::vector<rb::DevClock> hc(L->ndom);
   RB_CUDA(cudaMemcpyAsync(hc.data(), clocks, hc.size() * sizeof(rb::DevClock), cudaMemcpyDeviceToHost, s), "ens read");
   RB_CUDA(cudaStreamSynchronize(s), "rb_ensemble_read sync");
-  {
-    std::lock_guard<std::mutex> lock(g_ens_solo_mu);
-    auto it = g_ens_solo.find(ens);
-    if (it != g_ens_solo.end()) {
-      ens_regroup(it->second.li, hc);
-      ens_regroup(it->second.hllc, hc);
-    }
-  }
+  ens_regroup(ens, hc);
   for (int d = 0; d < L->ndom; d++) {
     out[d].t = hc[d].t;
     out[d].dt = hc[d].dt;

@@ -22,8 +22,6 @@
 
 namespace rb {
 
-constexpr double kEpsT = 1e-6;  // solver/scheduler.py:45 EPS_T
-
 // scheduler.py:48-72 fill_span
 __device__ __forceinline__ double fill_span(double span, double dt_raw) {
   if (!isfinite(span)) return dt_raw;

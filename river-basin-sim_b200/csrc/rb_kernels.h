@@ -49,6 +49,9 @@ struct DevClock {
   float stage32[4];
 };
 
+// A span ends when t >= t_target - kEpsT (solver/scheduler.py:45 EPS_T).
+constexpr double kEpsT = 1e-6;
+
 struct LiParams {
   int ny, nx;
   float dx32, dt32;
