@@ -271,6 +271,10 @@ int rb_ensemble_enqueue(const rb_ensemble_layout *L, void *ens, int32_t nsteps, 
  * RB_ERR_*). Every grouping computes the same bits: a graph captured under another one
  * stays right, and is only slower. */
 int rb_ensemble_route(const void *ens);
+/* Forbid grouping (0), from the next rb_ensemble_enqueue on, or allow it again, from the
+ * next rb_ensemble_set_targets or rb_ensemble_read on (the state after rb_ensemble_init).
+ * Host only. For timing the tile variants of the work-list, which grouped domains are not on. */
+int rb_ensemble_allow_groups(const void *ens, int32_t allow);
 /* Commit and read every domain's clock into out[ndom]. Synchronising. */
 int rb_ensemble_read(const rb_ensemble_layout *L, void *ens, rb_clock_state *out, void *stream);
 

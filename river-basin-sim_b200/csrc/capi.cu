@@ -742,6 +742,7 @@ int rb_clock_read(void* ws, void* stream, rb_clock_state* out) {
 struct EnsSolo {
   EnsRoute<rb::LiParams> li;
   EnsRoute<rb::HllcParams> hllc;
+  bool allow = true;  // rb_ensemble_allow_groups
 };
 static std::mutex g_ens_solo_mu;
 static std::unordered_map<const void*, EnsSolo> g_ens_solo;
@@ -749,7 +750,7 @@ static std::unordered_map<const void*, EnsSolo> g_ens_solo;
 static void ens_regroup(const void* ens, const std::vector<rb::DevClock>& clocks) {
   std::lock_guard<std::mutex> lock(g_ens_solo_mu);
   auto it = g_ens_solo.find(ens);
-  if (it == g_ens_solo.end()) return;
+  if (it == g_ens_solo.end() || !it->second.allow) return;
   ens_regroup(it->second.li, clocks);
   ens_regroup(it->second.hllc, clocks);
 }
@@ -996,6 +997,15 @@ int rb_ensemble_route(const void* ens) {
   auto it = g_ens_solo.find(ens);
   if (it == g_ens_solo.end()) return fail(RB_ERR_ARG, "rb_ensemble_route: the ensemble was not initialised");
   return (it->second.li.grouped ? 1 : 0) | (it->second.hllc.grouped ? 2 : 0);
+}
+
+int rb_ensemble_allow_groups(const void* ens, int32_t allow) {
+  std::lock_guard<std::mutex> lock(g_ens_solo_mu);
+  auto it = g_ens_solo.find(ens);
+  if (it == g_ens_solo.end()) return fail(RB_ERR_ARG, "rb_ensemble_allow_groups: the ensemble was not initialised");
+  it->second.allow = allow != 0;
+  if (allow == 0) it->second.li.grouped = it->second.hllc.grouped = false;
+  return RB_OK;
 }
 
 int rb_ensemble_read(const rb_ensemble_layout* L, void* ens, rb_clock_state* out, void* stream) {

@@ -125,6 +125,7 @@ SIGNATURES = {
     "rb_ensemble_set_targets": (ctypes.c_int, [ctypes.POINTER(EnsembleLayout), _P, _P, _P, _P]),
     "rb_ensemble_enqueue": (ctypes.c_int, [ctypes.POINTER(EnsembleLayout), _P, ctypes.c_int32, _P]),
     "rb_ensemble_route": (ctypes.c_int, [_P]),
+    "rb_ensemble_allow_groups": (ctypes.c_int, [_P, ctypes.c_int32]),
     "rb_ensemble_read": (ctypes.c_int, [ctypes.POINTER(EnsembleLayout), _P, _P, _P]),
     "rb_li_set_kernel_variant": (ctypes.c_int, [ctypes.c_int32]),
     "rb_li_kernel_variants": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int32)]),

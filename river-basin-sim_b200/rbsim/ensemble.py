@@ -95,6 +95,11 @@ class Ensemble:
         _lib.check(self._L.rb_ensemble_set_targets(ctypes.byref(self.layout), self._ws.data_ptr(), tt, mm,
                                                    self._stream()))  # fmt: skip
 
+    def allow_groups(self, allow: bool) -> None:
+        """Whether larger members may be stepped together (the default); forbidding it acts
+        at once, allowing it again at the next ``set_targets`` or ``read``."""
+        _lib.check(self._L.rb_ensemble_allow_groups(self._ws.data_ptr(), int(allow)))
+
     def replay(self) -> None:
         route = self._L.rb_ensemble_route(self._ws.data_ptr())
         if route < 0:
@@ -147,11 +152,15 @@ def autotune(make_ensemble, probe_replays: int = 2, candidates=None):
     computes the same bits, and a clock that restarted at the run's start would
     lay different steps toward its sync times. Build the production ensemble with
     ``t0 = times`` (the simulated time each member reached).
+
+    The candidates are timed without grouped launches: a group's members are not on the
+    work-list whose tiles are chosen here, until too few of them run and they return to it.
     """
     candidates = candidates or [(a, b) for a in LI_VARIANTS for b in HLLC_VARIANTS]
     timings, t0 = {}, None
     for li_v, hl_v in candidates:
         ens = make_ensemble(li_v, hl_v, t0)
+        ens.allow_groups(False)
         ens.replay()  # capture + first replay, untimed
         start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record()

@@ -44,3 +44,31 @@ def test_new_targets_group_only_domains_that_still_run(scheme):
     assert route() == 0
     ens.set_targets([2.0 * unit, 2.0 * unit, far])  # the large ones run again
     assert route() == bit
+
+
+@pytest.mark.parametrize("scheme", ["local_inertial", "hllc_fv"])
+def test_autotune_times_the_work_list_with_every_member_on_it(scheme):
+    """Its choice is of the work-list's tiles, which grouped members are not on."""
+    from rbsim.ensemble import Ensemble, autotune
+
+    hl = scheme == "hllc_fv"
+    members = [_member(scheme, ny, nx, k, "plain") for k, (ny, nx) in enumerate(SIDES[scheme])]
+    probes = []
+
+    def make(li_v, hl_v, t0):
+        e = Ensemble(members, [scheme] * 3, alpha=0.45 if hl else 0.7, dt_max=30.0, sync_times=[[1e6]] * 3,
+                     li_variant=li_v, hllc_variant=hl_v, graph_steps=2, t0=0.0 if t0 is None else t0)  # fmt: skip
+        e.set_targets(1e6)
+        probes.append(e)
+        return e
+
+    (li_v, hl_v), timings, t0 = autotune(make, probe_replays=1, candidates=[(0, 0), (3, 2)])
+    assert len(timings) == 2 and all(set(e._graphs) == {0} for e in probes)
+    run = make(li_v, hl_v, t0)
+    assert run._L.rb_ensemble_route(run._ws.data_ptr()) == (2 if hl else 1)
+    run.allow_groups(False)
+    run.set_targets(1e6)
+    assert run._L.rb_ensemble_route(run._ws.data_ptr()) == 0
+    run.allow_groups(True)
+    run.read()
+    assert run._L.rb_ensemble_route(run._ws.data_ptr()) == (2 if hl else 1)
