@@ -287,13 +287,13 @@ int rb_ensemble_read(const rb_ensemble_layout *L, void *ens, rb_clock_state *out
  * results; this is a speed knob only, read at each launch (a captured graph keeps
  * the variant it was captured with). The library starts with 6, which picks by the
  * domain's size what measured fastest on B200: 16 x 16, 32 x 16 or 32 x 32 tiles, or a
- * row-streaming kernel. */
+ * row-streaming kernel; 9 is its 32 x 32 tiles (640 threads) at any size. */
 int rb_hllc_set_kernel_variant(int32_t variant);
 int rb_hllc_kernel_variants(int32_t *count);
 /* The same for the local-inertial step (tile 32 x 16, 32 x 32, 64 x 16, 32 x 8, and
  * 32 x 16 held to 48 registers; a state with sub-grid channels always uses 32 x 16).
  * The library starts with 1, which picks by the domain's size: 16 x 16 or 32 x 32 tiles,
- * or a row-streaming kernel. */
+ * or a row-streaming kernel; 5 is its 32 x 32 tiles (512 threads) at any size. */
 int rb_li_set_kernel_variant(int32_t variant);
 int rb_li_kernel_variants(int32_t *count);
 

@@ -1437,7 +1437,7 @@ static cudaError_t launch_hllc_tma(const HllcParams& p, int stage, cudaStream_t 
 
 // Kernel variants of the single-domain stage: tile, block size, faces per work item,
 // load batching. All compute the same bits; they differ only in speed. The default (6)
-// chooses by the domain's size (hllc_default_tile, hllc_stream_takes); its 32 x 32 tiles
+// chooses by the domain's size (hllc_default_tile, hllc_stream_takes); its 32 x 32 tiles (9: at any size)
 // have 640 threads, two blocks and 40 warps per SM at 44-48 registers: fewer leave the
 // 2380 face work items of a tile an emptier last pass (3.7 passes of 640 threads, 4.6 of
 // 512), more spill. Staging interior tiles with tensor-memory copies is slower (7: one
@@ -1451,7 +1451,7 @@ struct HllcKernelVariant {
 static const HllcKernelVariant kHllcVariants[] = {
     {32, 16, 256, 1, 0}, {32, 16, 256, 1, 1}, {32, 16, 256, 3, 1},
     {32, 16, 256, 2, 1}, {32, 32, 512, 1, 1}, {64, 16, 512, 1, 1}, {32, 32, 640, 1, 1},
-    {32, 32, 640, 1, 2}, {32, 32, 512, 1, 3},
+    {32, 32, 640, 1, 2}, {32, 32, 512, 1, 3}, {32, 32, 640, 1, 1},
 };
 constexpr int kNumHllcVariants = (int)(sizeof(kHllcVariants) / sizeof(kHllcVariants[0]));
 constexpr int kDefaultHllcVariant = 6;
@@ -1519,6 +1519,7 @@ cudaError_t hllc_stage_launch_exact(const HllcParams& p, int stage, int variant,
     case 4: return launch_hllc<32, 32, 512, 1, 1>(p, stage, s);
     case 7: return launch_hllc_tma<32, 32, 640>(p, stage, s);
     case 8: return launch_hllc_tma<32, 32, 512, true>(p, stage, s);
+    case 9: return launch_hllc<32, 32, 640, 1, 1>(p, stage, s);
     default: break;
   }
   if (hllc_stream_takes(p)) return launch_hllc_stream(p, stage, s);

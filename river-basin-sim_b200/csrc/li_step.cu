@@ -709,11 +709,12 @@ static bool li_small(const LiParams& p) {
 // Tile variants of the single-domain step (sub-grid channels always use 32 x 16);
 // all compute the same bits. The default (1) chooses by the domain's size: 16 x 16
 // (li_small), 32 x 32 or the streaming kernel (li_stream_takes). Of the tiles 32 x 32 were
-// the fastest on B200 on the 2048^2 and 4096^2 rain-on-grid steps.
+// the fastest on B200 on the 2048^2 and 4096^2 rain-on-grid steps; 5 is those at any size.
 struct LiKernelVariant {
   int tx, ty, nt;
 };
-static const LiKernelVariant kLiVariants[] = {{32, 16, 256}, {32, 32, 512}, {64, 16, 512}, {32, 8, 256}, {32, 16, 256}};
+static const LiKernelVariant kLiVariants[] = {{32, 16, 256}, {32, 32, 512}, {64, 16, 512},
+                                              {32, 8, 256},  {32, 16, 256}, {32, 32, 512}};
 constexpr int kNumLiVariants = (int)(sizeof(kLiVariants) / sizeof(kLiVariants[0]));
 constexpr int kDefaultLiVariant = 1;
 #if !defined(RB_FAST_MATH)
@@ -743,6 +744,7 @@ cudaError_t li_step_launch_variant(const LiParams& p, int variant, cudaStream_t 
     case 2: return launch_li<64, 16, 512, false, 3>(p, s);
     case 3: return launch_li<32, 8, 256, false, 1>(p, s);
     case 4: return launch_li<32, 16, 256, false, 5>(p, s);  // at most 48 registers
+    case 5: return launch_li<32, 32, 512, false, 3>(p, s);
     default: break;
   }
   if (li_stream_takes(p)) return launch_li_stream(p, s);
