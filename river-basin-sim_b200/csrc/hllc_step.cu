@@ -1531,23 +1531,18 @@ cudaError_t hllc_stage_launch_exact(const HllcParams& p, int stage, int variant,
 }
 
 #if !defined(RB_FAST_MATH)
-// Tiles of the current variant (one ledger slot each); never more than the 32 x 8
-// tiling the workspace ledger is sized for.
-int hllc_tiles(int ny, int nx) { return hllc_tiles_of(g_hllc_variant.load(), ny, nx); }
-
+// Tiles of a variant on domains of at most kNoallocCells (one ledger slot each); never more
+// than the 32 x 8 tiling the workspace ledger is sized for.
 int hllc_tiles_of(int variant, int ny, int nx) {
   const bool known = variant >= 0 && variant < kNumHllcVariants;
   const HllcKernelVariant& v = kHllcVariants[known ? variant : kDefaultHllcVariant];
   int tx = v.tx, ty = v.ty;
-  const bool by_size = !known || variant == kDefaultHllcVariant;
-  if (by_size) {  // the default variant chooses its tile by the domain's size
+  if (!known || variant == kDefaultHllcVariant) {  // the default variant chooses its tile by the domain's size
     const int t = hllc_default_tile(ny, nx);
     tx = t == 0 ? 16 : 32;
     ty = t <= 1 ? 16 : 32;
   }
-  const int tiles = ((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
-  // its streaming kernel, in either arithmetic, has a slot per block
-  return by_size && hllc_stream_fits(ny, nx) ? std::max(tiles, hllc_stream_blocks(ny, nx)) : tiles;
+  return ((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
 }
 
 // Ensemble: one Heun stage over the (domain, local tile) work-list of every HLLC

@@ -18,7 +18,7 @@
 #pragma once
 
 constexpr int kHllcHalo = 3;
-static_assert(kHllcStreamCols == 32 - 2 * kHllcHalo, "columns a strip stores");
+constexpr int kHllcStreamCols = 32 - 2 * kHllcHalo;  // columns a strip stores
 
 // A warp's staging area: the row in use and the one on its way, each lane's word of
 // every array its iteration reads. Arrays: h, hu, hv, z of row r; of row r - 3 the
@@ -417,6 +417,17 @@ __global__ void __launch_bounds__(32, kHllcStreamWarps) hllc_stream_kernel(const
                                 rows, ring);
 }
 
+// Rows a warp walks: two waves of the warps the GPU holds, within 11 .. 48: three rows
+// above and below a chunk are overhead, and with one long wave the domain's edge strips,
+// which check bounds, end last (2048^2 dam break, fast, us per step: 196 / 190 / 191 / 228
+// for 19 / 28 / 35 / 48 rows).
+static int hllc_stream_rows(int ny, int nx) {
+  constexpr long long kWarps = 2LL * 148 * kHllcStreamWarps;
+  const long long strips = (nx + kHllcStreamCols - 1) / kHllcStreamCols;
+  const long long rows = (ny * strips + kWarps - 1) / kWarps;
+  return (int)(rows < 11 ? 11 : (rows > 48 ? 48 : rows));
+}
+
 static cudaError_t launch_hllc_stream(const HllcParams& p, int stage, cudaStream_t s) {
   const int rows = hllc_stream_rows(p.ny, p.nx);
   const dim3 grid((p.nx + kHllcStreamCols - 1) / kHllcStreamCols, (p.ny + rows - 1) / rows), block(32);
@@ -426,7 +437,7 @@ static cudaError_t launch_hllc_stream(const HllcParams& p, int stage, cudaStream
              : launch_chain(hllc_stream_kernel<2, 0>, grid, block, 0, s, p, rows);
 }
 
-// Whether the streaming kernel takes this domain (with hllc_stream_fits). Below these sizes
+// Whether the streaming kernel takes this domain. Below these sizes
 // the 32 x 32 tiles are as fast or faster: a warp walks its rows one after another, and a
 // small domain has too few warps to hide that; on a narrow one the strips at the west and
 // east edge, which check bounds, are too many (us per step, tiles / streaming -- fast dam
@@ -438,8 +449,14 @@ constexpr long long kHllcStreamCells = 1500000;
 #else
 constexpr long long kHllcStreamCells = 2300000;
 #endif
+static_assert(kHllcStreamCells > kNoallocCells, "a streamed domain has a ledger slot per strip and chunk");
 static bool hllc_stream_takes(const HllcParams& p) {
-  return (long long)p.ny * p.nx >= kHllcStreamCells && p.nx >= 30 * kHllcStreamCols && hllc_stream_fits(p.ny, p.nx);
+  if ((long long)p.ny * p.nx < kHllcStreamCells || p.nx < 30 * kHllcStreamCols) return false;
+  // a ledger slot (32 x 8 cells) per strip and chunk: all but narrow and flat domains have them
+  const int rows = hllc_stream_rows(p.ny, p.nx);
+  const long long blocks = (long long)((p.nx + kHllcStreamCols - 1) / kHllcStreamCols) * ((p.ny + rows - 1) / rows);
+  if (blocks > (long long)((p.nx + 31) / 32) * ((p.ny + 7) / 8)) return false;
+  return (p.ny + rows - 1) / rows <= 65535 && (long long)(rows + 16) * p.nx < (1LL << 31);
 }
 
 #if !defined(RB_FAST_MATH)

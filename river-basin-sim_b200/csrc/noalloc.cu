@@ -35,7 +35,7 @@
 
 namespace {
 
-constexpr int64_t kMaxCells = int64_t(1) << 20;
+constexpr int64_t kMaxCells = rb::kNoallocCells;
 constexpr int64_t kMaxTiles = int64_t(1) << 17;  // ledger slots; any shape within kMaxCells needs fewer
 constexpr size_t kPlane = (size_t)kMaxCells * sizeof(float);
 constexpr size_t kLedgerOff = rb::WS_LEDGER;

@@ -97,31 +97,6 @@ struct HllcParams {
   unsigned int *err;
 };
 
-// The row-streaming HLLC stage kernel's split (hllc_stream.cuh), the same in both
-// arithmetics: columns a warp's strip stores, rows a warp walks, blocks (one ledger slot
-// each) of a domain, and whether a domain's strips fit the ledger (a slot per 32 x 8
-// cells: all but narrow and flat domains do), the grid and 32-bit row offsets.
-constexpr int kHllcStreamCols = 26;
-// Two waves of the 16 warps an SM holds, within 11 .. 48 rows: three rows above and below
-// a chunk are overhead, and with one long wave the domain's edge strips, which check
-// bounds, end last (2048^2 dam break, fast, us per step: 196 / 190 / 191 / 228 for 19 / 28 /
-// 35 / 48 rows).
-inline int hllc_stream_rows(int ny, int nx) {
-  const long long strips = (nx + kHllcStreamCols - 1) / kHllcStreamCols;
-  const long long rows = (ny * strips + 2 * 148 * 16 - 1) / (2 * 148 * 16);
-  return (int)(rows < 11 ? 11 : (rows > 48 ? 48 : rows));
-}
-inline int hllc_stream_blocks(int ny, int nx) {
-  const int rows = hllc_stream_rows(ny, nx);
-  return ((nx + kHllcStreamCols - 1) / kHllcStreamCols) * ((ny + rows - 1) / rows);
-}
-inline bool hllc_stream_fits(int ny, int nx) {
-  const int rows = hllc_stream_rows(ny, nx);
-  const long long blocks = (long long)((nx + kHllcStreamCols - 1) / kHllcStreamCols) * ((ny + rows - 1) / rows);
-  return blocks <= (long long)((nx + 31) / 32) * ((ny + 7) / 8) && (ny + rows - 1) / rows <= 65535 &&
-         (long long)(rows + 16) * nx < (1LL << 31);
-}
-
 // Domains of an ensemble that one launch of a row-streaming kernel steps together: their
 // parameters by value, as in a domain's own launch, domain d's strips and chunks being
 // blocks first[d] .. first[d + 1].
@@ -158,6 +133,10 @@ struct HllcMaps {
   TileMap h[2], hu[2], hv[2], z, h1, hu1, hv1;
 };
 
+// The most cells rb_hllc_step_noalloc takes. It clears and sums a ledger slot per tile of
+// hllc_tiles_of, so that no larger split may step a domain of this size.
+constexpr long long kNoallocCells = 1LL << 20;
+
 cudaError_t li_step_launch(const LiParams& p, cudaStream_t s);
 cudaError_t li_step_launch_variant(const LiParams& p, int variant, cudaStream_t s);
 int li_current_variant();
@@ -191,7 +170,6 @@ bool ens_li_stream_fits(const LiParams& p);
 bool ens_hllc_stream_fits(const HllcParams& p);
 cudaError_t ens_li_stream_launch(const LiParams* p, int n, cudaStream_t s);
 cudaError_t ens_hllc_stream_launch(const HllcParams* p, int n, int stage, cudaStream_t s);
-int hllc_tiles(int ny, int nx);
 // The HLLC stage-kernel variant in force now; the launch and tile count of one call
 // can take it once, so a concurrent rb_hllc_set_kernel_variant cannot split them.
 int hllc_current_variant();
