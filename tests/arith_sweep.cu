@@ -1,7 +1,8 @@
 // arith_sweep.cu -- the step kernels' hand-written arithmetic (csrc/rb_common.cuh,
-// csrc/pair.cuh) over the ranges its comments state. Compiled by test_gpu_arith_sweep.py
+// csrc/pair.cuh, csrc/hllc_face.cuh) over the ranges its comments state. Compiled by test_gpu_arith_sweep.py
 // once per arithmetic, with that build's flags. A check maps an index to operands and says
 // whether what it got is what it should be.
+#include <cfloat>
 #include <cmath>
 
 #include "rb_common.cuh"
@@ -9,6 +10,8 @@
 namespace rb {
 RB_ARITH_BEGIN
 #include "pair.cuh"
+#include "warp_stream.cuh"
+#include "hllc_face.cuh"
 
 using u64 = unsigned long long;
 
@@ -165,6 +168,87 @@ struct Slope {
     return same(face_slope(de, dx, slope_rcp(dx)), __fdiv_rn(de, dx));
   }
 };
+
+// Depths, velocities and momenta as states hold them and beyond: zeros, the dry limit,
+// ordinary values, and any bits (subnormals, infinities, not a number).
+__device__ __forceinline__ float some_depth(u64 r) {
+  const unsigned m = (unsigned)(r >> 32);
+  switch (r & 15) {
+    case 0: return 0.0f;
+    case 1: return flt(bits(kHDry) - 2 + (m & 3));  // either side of the dry limit
+    case 2: return flt(m & 0x7fffffffu);
+    case 3: return flt(m);
+    case 4: return in_binade((int)(r >> 8) % 24 + 10, m);  // 2^10 .. 2^33
+    default: return in_binade((int)((r >> 8) % 16) - 10, m);  // 2^-10 .. 2^5
+  }
+}
+__device__ __forceinline__ float some_speed(u64 r) {
+  const unsigned m = (unsigned)(r >> 32), sign = m & 0x80000000u;
+  switch (r & 15) {
+    case 0: return flt(sign);
+    case 1: return flt(m);
+    case 2: return flt(sign | bits(in_binade((int)((r >> 8) % 120) - 60, m)));
+    default: return flt(sign | bits(in_binade((int)((r >> 8) % 20) - 16, m)));  // 2^-16 .. 2^3
+  }
+}
+
+// The Riemann solve, guarded scalar and packed, against the general form. Half of the faces
+// run close to critical (a wave speed near zero) or nearly at rest with equal sides.
+struct Riemann {
+  static u64 count() { return 1ull << 28; }
+  struct Face {
+    float hl, ul, vl, hr, ur, vr;
+  };
+  __device__ static Face face(u64 r) {
+    const u64 a = mix(r), b = mix(a), c = mix(b), d = mix(c), e = mix(d), g = mix(e);
+    Face f{some_depth(a), some_speed(b), some_speed(c), some_depth(d), some_speed(e), some_speed(g)};
+    if (r & 1) {
+      if (r & 2) f.hr = f.hl;
+      if (r & 4) f.ur = f.ul;
+      const int off = (int)(g >> 40 & 7) - 3;
+      if ((r & 24) == 8) f.ul = flt(bits(sqrtf(kG * fmaxf(f.hl, 0.0f))) + off);
+      if ((r & 24) == 16) f.ur = -flt(bits(sqrtf(kG * fmaxf(f.hr, 0.0f))) + off);
+    }
+    return f;
+  }
+  __device__ static bool equal(const Face& f, float f0, float f1, float f2) {
+    float w0, w1, w2;
+    hllc_flux_any(f.hl, f.ul, f.vl, f.hr, f.ur, f.vr, w0, w1, w2);
+    return same(f0, w0) && same(f1, w1) && same(f2, w2);
+  }
+  __device__ bool operator()(u64 k, Operands& o) const {
+    const Face f = face(mix(2 * k)), h = face(mix(2 * k + 1));
+    o = Operands{f.hl, f.hr};
+    float f0, f1, f2;
+    hllc_flux(f.hl, f.ul, f.vl, f.hr, f.ur, f.vr, f0, f1, f2);
+    F2 p0, p1, p2;
+    bool odd = false;
+    hllc_near2(F2{f.hl, h.hl}, F2{f.ul, h.ul}, F2{f.vl, h.vl}, F2{f.hr, h.hr}, F2{f.ur, h.ur}, F2{f.vr, h.vr}, p0, p1,
+               p2, odd);
+    return equal(f, f0, f1, f2) && (odd || (equal(f, p0.x, p1.x, p2.x) && equal(h, p0.y, p1.y, p2.y)));
+  }
+};
+
+// A cell's primitives, friction and wave speed, guarded, against the general forms.
+struct CellValues {
+  static u64 count() { return 1ull << 28; }
+  __device__ bool operator()(u64 k, Operands& o) const {
+    const u64 a = mix(k), b = mix(a), c = mix(b), d = mix(c);
+    const float h = some_depth(a), hu = some_speed(b), hv = (c & 0x300) == 0 ? hu : some_speed(c);
+    o = Operands{h, hu};
+    float u, v, wu, wv;
+    primitives(h, hu, hv, u, v);
+    primitives_any(h, hu, hv, wu, wv);
+    const bool wet = h > kHDry;
+    const float n = (d & 15) == 0 ? 0.0f : (d & 15) == 1 ? flt((unsigned)(d >> 32)) : (float)(d >> 8 & 1023) * 0.0005f;
+    const float gdt = kG * in_binade((int)(d >> 20 & 15) - 8, (unsigned)(d >> 32));
+    float qu = hu, qv = hv, gu = hu, gv = hv;
+    hllc_friction<false>(h, wet, gdt, n, qu, qv);
+    friction_any(h, wet, gdt, n, gu, gv);
+    return same(u, wu) && same(v, wv) && same(qu, gu) && same(qv, gv) &&
+           same(wave_speed<false>(h, hu, hv), wave_speed_any(h, hu, hv));
+  }
+};
 #else
 // The bounds are those of the units' documentation (reciprocal: 1 ulp; square root: 2^-23;
 // logarithm: 2^-22 of max(1, |result|); exponential: 2 ulp of the rounded result) and of
@@ -248,6 +332,8 @@ RB_SWEEP(over_g, OverG)
 RB_SWEEP(denominator, Denominator)
 RB_SWEEP(manning, Manning)
 RB_SWEEP(slope, Slope)
+RB_SWEEP(riemann, Riemann)
+RB_SWEEP(cell_values, CellValues)
 #endif
 
 RB_ARITH_END

@@ -21,7 +21,8 @@ pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CHECKS = {
-    "exact": ["reciprocal", "root", "power", "over_g", "quotient", "denominator", "manning", "slope"],
+    "exact": ["reciprocal", "root", "power", "over_g", "quotient", "denominator", "manning", "slope", "riemann",
+              "cell_values"],
     "fast": ["quotient", "root", "power"],
 }
 
