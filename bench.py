@@ -10,7 +10,7 @@ here.
 
 * ``value``: whole-job cell-updates per second with the state resident on the
   device: K steps on the device-resident clock (dt, fill_span and rain gating in
-  a one-thread plan kernel), replayed as one CUDA graph, timed with CUDA events
+  a one-warp plan kernel), replayed as one CUDA graph, timed with CUDA events
   between a barrier + synchronize on each side (max over ranks).
 * ``e2e``: the same metric through the public API from host memory: the bed and
   initial depth are copied in from pinned host buffers (State.from_bed), K steps
@@ -20,7 +20,7 @@ here.
   every step as the reference does.
 * ``roofline``: the step's kernels against the measured HBM copy bandwidth, from
   algorithmic bytes (32 B per cell-step: read h, hu, hv, z, n; write h, hu, hv) over
-  the CUDA-event time of the timed replay itself (which also holds the one-thread
+  the CUDA-event time of the timed replay itself (which also holds the one-warp
   plan kernel of each step, so the figure is a lower bound for the stage pair);
   ``launched_one_by_one`` times each stage kernel with events around single launches
   as a cross-check.
@@ -62,10 +62,11 @@ T_END = 30.0  # simulated horizon of the dam-break configuration
 BYTES_PER_CELL_STEP = 32  # read h, hu, hv, z, n (20 B) + write h, hu, hv (12 B)
 # DRAM bytes (read + write) of one step's two stage launches in one ncu capture of this
 # workload (2048^2 dam break, streaming kernels, fast build, stage 1 + stage 2): 83.3 MB +
-# 178.0 MB (the exact build: 83.4 + 175.6 MB).
+# 178.0 MB (the exact build on the 2048^2 lake: 83.4 + 175.6 MB).
 NCU_DRAM_BYTES_PER_STEP = 261.4e6
-# The stage kernels are issue-bound: share of issue slots busy in the same capture
-# (fast build: stage 1 72.5 %, stage 2 68.7 %; exact: 73.0 %, 71.9 %).
+# The stage kernels are bound by issue and by latency at four warps a scheduler: share of
+# issue slots busy in the same captures (fast dam break: stage 1 72.5 %, stage 2 68.7 %;
+# exact lake: 73.0 %, 71.9 %).
 NCU_ISSUE_ACTIVE = (0.725, 0.687)
 WORKLOAD = "hllc_dambreak_2048x2048"
 BUILDS = {
@@ -405,7 +406,7 @@ def main(argv=None) -> int:
     if rank == 0:
         pk = peaks()
         # roofline from the timed region itself: the step's algorithmic bytes over the
-        # replayed step's event time (which also holds the one-thread plan kernel, so
+        # replayed step's event time (which also holds the one-warp plan kernel, so
         # this is a lower bound for the two stage kernels)
         achieved = BYTES_PER_CELL_STEP * cells / (ms / K / 1e3) / 1e9
         mean_kernel_ms = statistics.mean(a + b for a, b in zip(stage1_ms, stage2_ms, strict=True))
@@ -426,7 +427,7 @@ def main(argv=None) -> int:
                                          "ncu capture of this workload; the algorithmic bytes per step are 134 MB",
                          "peak_source": pk["source"],
                          "timing": "CUDA events around the timed replay of K steps (stage 1 + stage 2 + the "
-                                   "one-thread plan kernel per step): a lower bound for the stage pair",
+                                   "one-warp plan kernel per step): a lower bound for the stage pair",
                          "issue_bound": {"issue_slots_busy_stage1": NCU_ISSUE_ACTIVE[0],
                                          "issue_slots_busy_stage2": NCU_ISSUE_ACTIVE[1],
                                          "source": "the same ncu capture"},

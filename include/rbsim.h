@@ -164,7 +164,7 @@ int rb_read_device_error(void *ws, void *stream, uint32_t *err_out);
 
 /* --- device-resident clock ----------------------------------------------------
  * The run loop of solver/run.py:369-388 with the scheduler of
- * solver/scheduler.py:171-246, moved onto the device: a one-thread plan kernel
+ * solver/scheduler.py:171-246, moved onto the device: a one-warp plan kernel
  * turns the max the previous step folded into the clock into compute_dt's dt,
  * clamps it with fill_span to the next sync time, gates the rain and banks its
  * volume, all in float64 in the reference's operation order, so K steps run

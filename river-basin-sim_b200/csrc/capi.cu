@@ -201,12 +201,13 @@ struct EnsRoute {
 // fastest (its rule for one domain), but a domain's step takes a warp's walk down a chunk
 // however small the domain, so that it pays only while the domains still running hold
 // `cells`, and for domains of at least `tiles`; smaller ones join when they are at most a
-// tenth of it, which saves their own launch. Measured on B200 (us per step of n domains of
-// side x side, work-list or own launches / grouped): LI 16 x 256 38.1 / 39.2, 64 x 256
-// 132 / 150, 25 x 400 130 / 120, 4 x 512 37.3 / 35.4, 10 x 600 112 / 87, 6 x 860 133 / 113,
-// 4 x 1000 119 / 98; HLLC 64 x 256 366 / 535, 25 x 400 362 / 417, 3 x 1000 248 / 241,
-// 10 x 600 316 / 292, 6 x 860 378 / 333, 4 x 1000 331 / 306. One domain left of a group:
-// LI 400 15.5 / 33, HLLC 400 33 / 81.
+// tenth of it, which saves their own launch. Measured on B200 before the kernels packed
+// their faces, which made the grouped side quicker (us per step of n domains of side x
+// side, work-list or own launches / grouped): LI 16 x 256 38.1 / 39.2, 64 x 256 132 / 150,
+// 25 x 400 130 / 120, 4 x 512 37.3 / 35.4, 10 x 600 112 / 87, 6 x 860 133 / 113, 4 x 1000
+// 119 / 98; HLLC 64 x 256 366 / 535, 25 x 400 362 / 417, 3 x 1000 248 / 241, 10 x 600 316 /
+// 292, 6 x 860 378 / 333, 4 x 1000 331 / 306. One domain left of a group: LI 400 15.5 / 33,
+// HLLC 400 33 / 81.
 struct EnsRowRule {
   int64_t tiles;
   long long cells;

@@ -4,7 +4,7 @@
 // scheme.compute_dt reads max(h) (or the max wave speed) back to the host, the
 // scheduler (solver/scheduler.py:171-246) clamps it with fill_span to the next
 // sync point, the run loop gates rain on `t < rain_duration - EPS_T` and banks
-// the rain volume in the float64 ledger. Here one single-thread "plan" kernel
+// the rain volume in the float64 ledger. Here one "plan" kernel of a single warp
 // does all of that in float64 on the device, reading the max the previous step
 // kernel folded into the clock, so K steps run back to back (and can be captured
 // in a CUDA graph) with no host round trip. Same float64 operations in the same

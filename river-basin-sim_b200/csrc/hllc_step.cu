@@ -1097,8 +1097,8 @@ static cudaError_t launch_hllc_tma(const HllcParams& p, int stage, cudaStream_t 
 
 // Kernel variants of the single-domain stage: tile, block size, faces per work item,
 // load batching. All compute the same bits; they differ only in speed. The default (6)
-// chooses by the domain's size (hllc_default_tile, hllc_stream_takes); its 32 x 32 tiles (9: at any size)
-// have 640 threads, two blocks and 40 warps per SM at 44-48 registers: fewer leave the
+// chooses by the domain's size (hllc_default_tile, hllc_stream_takes); its 32 x 32 tiles
+// (9: at any size) have 640 threads, two blocks and 40 warps per SM at 44-48 registers: fewer leave the
 // 2380 face work items of a tile an emptier last pass (3.7 passes of 640 threads, 4.6 of
 // 512), more spill. Staging interior tiles with tensor-memory copies is slower (7: one
 // tile a block, by 1 %; 8: one resident block of 512 threads per slot walking the tiles

@@ -437,13 +437,14 @@ static cudaError_t launch_hllc_stream(const HllcParams& p, int stage, cudaStream
              : launch_chain(hllc_stream_kernel<2, 0>, grid, block, 0, s, p, rows);
 }
 
-// Whether the streaming kernel takes this domain. Below these sizes
-// the 32 x 32 tiles are as fast or faster: a warp walks its rows one after another, and a
-// small domain has too few warps to hide that; on a narrow one the strips at the west and
-// east edge, which check bounds, are too many (us per step, tiles / streaming -- fast dam
+// Whether the streaming kernel takes this domain. A warp walks its rows one after another,
+// and a small domain has too few warps to hide that; on a narrow one the strips at the west
+// and east edge, which check bounds, are too many (us per step, tiles / streaming -- fast dam
 // breaks: 1024^2 65.6 / 67.4, 1200^2 87.8 / 82.7, 2048^2 265 / 178; exact lakes: 1024^2 87 /
 // 100, 1200^2 116 / 122, 1448^2 164 / 157, 2600 x 800 161 / 163, 1600^2 198 / 185; exact
-// dam break, 2048^2 306 / 246).
+// dam break, 2048^2 306 / 246). The limits lie above the largest domain on which the tiles
+// won (fast 1024^2; exact 2600 x 800, 2.08 M cells) and not at the crossover of square ones,
+// which is lower: a fast 1200^2 and an exact 1448^2 would gain 6 % and 4 % by streaming.
 #if defined(RB_FAST_MATH)
 constexpr long long kHllcStreamCells = 1500000;
 #else

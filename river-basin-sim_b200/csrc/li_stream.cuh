@@ -408,13 +408,15 @@ static int li_stream_rows(int ny, int nx) {
   return (int)(rows < 8 ? 8 : (rows > 48 ? 48 : rows));
 }
 
-// Whether the streaming kernel takes this domain. Below kLiStreamCells the 32 x 32 tiles
-// are as fast or faster, since a warp walks its rows one after another and a small domain
-// has too few warps to hide that (measured us per step, tiles / streaming -- exact: 1024^2
-// 32.7 / 32.9, 1200^2 42.2 / 39.5, 1531 x 1017 with rain field and infiltration 47.5 / 48.1,
-// 1380^2 53.1 / 48.6, 2048^2 118 / 92; fast: 512^2 18.0 / 18.2, 1024^2 28.9 / 22.9, 1531 x
-// 1017 39.4 / 33.2, 2048^2 89.6 / 54.3, 4096^2 322 / 170). The ledger has a slot per 32 x 8
-// cells, enough for one per strip and chunk except on narrow or flat domains.
+// Whether the streaming kernel takes this domain. A warp walks its rows one after another,
+// and a small domain has too few warps to hide that (us per step, tiles / streaming --
+// exact: 1024^2 32.7 / 32.9, 1200^2 42.2 / 39.5, 1531 x 1017 with rain field and
+// infiltration 47.5 / 48.1, 1380^2 53.1 / 48.6, 2048^2 118 / 92; fast: 512^2 18.0 / 18.2,
+// 1024^2 28.9 / 22.9, 1531 x 1017 39.4 / 33.2, 2048^2 89.6 / 54.3, 4096^2 322 / 170). One
+// limit serves all sources and lies above the largest domain on which the tiles won, that
+// with rain field and infiltration (1.56 M cells); a plain 1200^2 would gain 6 % by
+// streaming. The ledger has a slot per 32 x 8 cells, enough for one per strip and chunk
+// except on narrow or flat domains.
 #if defined(RB_FAST_MATH)
 constexpr long long kLiStreamCells = 400000;
 #else

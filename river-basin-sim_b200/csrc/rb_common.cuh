@@ -6,10 +6,10 @@
 //    expression order (identical to the CPU oracle); the fractional powers come
 //    from include/rb_detmath.h;
 //  * fast (csrc/fast/, RB_FAST_MATH defined, everything in namespace rb::fast):
-//    contracted multiply-adds, the hardware's approximate division and square root
-//    and __powf for the fractional powers -- the arithmetic of a GPU build of the
-//    reference, held to the solver tolerance instead of bit equality. Compensated
-//    (Kahan) additions stay explicit IEEE adds in both.
+//    contracted multiply-adds and the hardware's approximate division, square root
+//    and powers -- the arithmetic of a GPU build of the reference, held to the solver
+//    tolerance instead of bit equality. Compensated (Kahan) additions stay explicit
+//    IEEE adds in both.
 // `rmax/rmin/rclamp` are the scalar builtins of the reference's kernel language
 // (a > b ? a : b, a < b ? a : b, min(max(lo,x),hi)), which differ from
 // fmaxf/fminf on signed zeros.
@@ -352,7 +352,7 @@ RB_ARITH_END
 // done. Triggered at its start instead, the next grid's blocks take slots beside it and are
 // packed onto few SMs (us per step, trigger at the start / at the end: 512^2 rain-on-grid
 // 20.7 / 16.1, 256^2 dam break 30.8 / 23.1, 2048^2 dam break fast 192.1 / 190.3). The
-// one-thread plan triggers at its start. A kernel launched without the attribute does not
+// plan, one warp, triggers at its start. A kernel launched without the attribute does not
 // start early, and for it the wait returns at once.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

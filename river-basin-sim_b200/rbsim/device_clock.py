@@ -2,7 +2,7 @@
 
 The reference run loop (solver/run.py:369-388) reads a float back from the device
 every step (``compute_dt``) and clamps it on the host (solver/scheduler.py). Here
-the same float64 arithmetic runs in a one-thread plan kernel on the device
+the same float64 arithmetic runs in a one-warp plan kernel on the device
 (librbsim ``rb_clock_plan``), the step kernels read their dt from it, and a span of
 ``graph_steps`` steps is captured once into a CUDA graph and replayed. The host only
 looks at the clock between replays, and only to ask "has the span's target been
